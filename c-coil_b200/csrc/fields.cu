@@ -110,10 +110,23 @@ __global__ void boundedWaitKernel(long long limit, int *status)
 
 #include "integrands64.cuh"
 
-// 6 CTAs of 128 threads per SM (80 registers; measured best on B200)
+// CTAs of 128 threads per SM that the register allocation targets.  The FP64
+// pipe bounds these kernels (80-90 % busy by its measured rate); what keeps it
+// fed is four nodes in flight per thread (kUnroll64) without spills, rather than
+// more warps: 128 coils at 2^17 points take A 36.8, B 29.2 ms at 4 CTAs (122-124
+// registers) against 39.0 and 30.5 at 5 and 37.5 and 29.6 at 3, G 53.3 ms at 3
+// (158 registers) against 55.3 at 4 and 52.9 at 2.  With the IEEE root and
+// division of the compiler the same launches took 69.4, 49.8 and 95.0 ms.
 #ifndef CCOIL_FP64_MIN_BLOCKS
-#define CCOIL_FP64_MIN_BLOCKS 6
+#define CCOIL_FP64_MIN_BLOCKS 4
 #endif
+#ifndef CCOIL_FP64_MIN_BLOCKS_G
+#define CCOIL_FP64_MIN_BLOCKS_G 3
+#endif
+constexpr int fp64MinBlocks(int field)
+{
+    return field == CCOIL_FIELD_G ? CCOIL_FP64_MIN_BLOCKS_G : CCOIL_FP64_MIN_BLOCKS;
+}
 // 1: segments staged into shared memory (double-buffered bulk copies, one CTA
 // barrier per segment); 0 (default): each warp reads the tables from global
 // memory through L1, with no barrier between warps
@@ -122,7 +135,7 @@ __global__ void boundedWaitKernel(long long limit, int *status)
 #endif
 
 template <int FIELD, int LANES>
-__global__ void __launch_bounds__(128, CCOIL_FP64_MIN_BLOCKS) fieldsKernel64(const unsigned char *__restrict__ blob,
+__global__ void __launch_bounds__(128, fp64MinBlocks(FIELD)) fieldsKernel64(const unsigned char *__restrict__ blob,
                                                       const SegmentDesc *__restrict__ segs, int nseg,
                                                       const double *__restrict__ points, long long npts,
                                                       double *__restrict__ out)

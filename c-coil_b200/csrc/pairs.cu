@@ -412,8 +412,16 @@ __device__ __forceinline__ void transformDerivatives(double yA, double zA, doubl
     dTz[6] = sY * sZ;          dTz[7] = sY * cZ;          dTz[8] = 0.0;
 }
 
+// CTAs per SM the register allocation targets, FP64 kernels: as the field
+// kernels', four nodes in flight per thread without spills (M 128 registers, F/T
+// 168).  2^15 arrangements of the 408 x 374-node pair: M 19.3 ms at 4 (19.8 at 5,
+// 19.2 at 3), F/T 12.9 ms at 3 (13.1 at 4, 13.6 at 2); with the compiler's IEEE
+// root and division 35.0 and 21.3 ms
 #ifndef CCOIL_PAIR_MIN_BLOCKS
-#define CCOIL_PAIR_MIN_BLOCKS 6
+#define CCOIL_PAIR_MIN_BLOCKS 4
+#endif
+#ifndef CCOIL_PAIR_MIN_BLOCKS_FT
+#define CCOIL_PAIR_MIN_BLOCKS_FT 3
 #endif
 // the same for the FP32 variants (M and F/T, packed integrands with the
 // subtracted mirror differences): 9 measured best against 6 (M 69.6 and
@@ -541,7 +549,7 @@ __device__ __noinline__ double2 pairB32(const SegmentHeader &h, const double2 *t
 // cancellation magnifies.
 template <int QTY, bool FP32, bool REFINE = false>
 __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS : CCOIL_PAIR32_MIN_BLOCKS)
-                                               : CCOIL_PAIR_MIN_BLOCKS)
+                                               : (QTY == 1 ? CCOIL_PAIR_MIN_BLOCKS_FT : CCOIL_PAIR_MIN_BLOCKS))
     pairKernel64(const unsigned char *__restrict__ blob, const long long *__restrict__ primOffsets, int nprim,
                  const double *__restrict__ primPoses, const double *__restrict__ secPoses, long long count,
                  double *__restrict__ out, unsigned long long *__restrict__ zAxisCount, int stagedBytes,

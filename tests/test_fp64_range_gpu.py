@@ -1,0 +1,52 @@
+"""FP64 integrands at the edges of the range in which they take their own roots
+and quotients ([1e-36, 1e36] for squared distances; IEEE operations beyond):
+geometries scaled across it, and points on a winding's own radius.  Bar: the
+parity bar of test_fields_gpu.py, 1e-12 per point against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import gradient_band, rel_err
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def coils_and_points(ccoil, scale, seed):
+    from ccoil_b200 import workloads
+    rows = workloads.coil_rows_mixed(8, seed=seed)
+    rows[:, 0:3] *= scale
+    rows[:, 6:9] *= scale
+    pts = workloads.points_cube(97, seed=seed + 1) * scale
+    return rows, workloads.coils_from_rows(rows, 4.0), pts
+
+
+# squared distances span about 1e-4..10 times scale^2: inside the range, across
+# its lower and upper ends, and outside it
+@pytest.mark.parametrize("scale", [1.0, 1e-10, 3e-18, 1e-21, 1e10, 3e17, 1e21])
+@pytest.mark.parametrize("field", [0, 1, 3])
+def test_scaled_geometry_against_oracle(ccoil, oracle, scale, field):
+    rows, coils, pts = coils_and_points(ccoil, scale, seed=31)
+    group = ccoil.CoilGroup(coils, ccoil.PrecisionFactor(4.0))
+    plan = group.plan(field)
+    got = plan(pts)
+    plan.close()
+    e = rel_err(got, oracle.group_fields(rows, pts, field, pf=4.0))
+    if field == 3:
+        e = e[~gradient_band(rows, pts)]
+    assert np.all(np.isfinite(got)) and e.max() < TOL, e.max()
+
+
+@pytest.mark.parametrize("field", [0, 1])
+@pytest.mark.parametrize("lanes", [1, 8])
+def test_points_on_the_winding_radius(ccoil, oracle, field, lanes):
+    # r equals the node radius: the smallest squared distance bound is exactly zero
+    row = np.array([0.1, 0.0, 0.08, 40, 2.0, 50.0, 0.0, 0.0, 0.0, 0.0, 0.0])
+    z = np.array([0.0, 0.02, -0.039, 0.04, 0.0401, -0.3])
+    pts = np.stack([np.full_like(z, 0.1), np.zeros_like(z), z], axis=1)
+    coil = ccoil.Coil(0.1, 0.0, 0.08, 40, 2.0)
+    plan = ccoil.FieldPlan([coil.struct()], field)
+    got = plan(pts, lanes=lanes)
+    plan.close()
+    e = rel_err(got, oracle.coil_fields(row, pts, field, pf=5.0))
+    assert e.max() < TOL, e.max()
