@@ -437,6 +437,13 @@ __device__ __forceinline__ void transformDerivatives(double yA, double zA, doubl
 #ifndef CCOIL_PAIR32R_MIN_BLOCKS
 #define CCOIL_PAIR32R_MIN_BLOCKS 9
 #endif
+constexpr int pairMinBlocks(int qty, bool fp32, bool refine)
+{
+    return refine ? CCOIL_PAIR32R_MIN_BLOCKS
+           : fp32 ? CCOIL_PAIR32_MIN_BLOCKS
+           : qty == 1 ? CCOIL_PAIR_MIN_BLOCKS_FT
+                      : CCOIL_PAIR_MIN_BLOCKS;
+}
 // FP32_REFINED arrangements: the largest scratch of node contributions (the
 // grid shrinks to fit it)
 constexpr size_t kPairRefineScratchBytes = size_t(1) << 30;
@@ -444,6 +451,21 @@ constexpr size_t kPairRefineScratchBytes = size_t(1) << 30;
 #ifndef CCOIL_PAIR_STAGE_MAX_BYTES
 #define CCOIL_PAIR_STAGE_MAX_BYTES (48 * 1024)
 #endif
+
+// units per arrangement: groups of primaries x ranges of secondary nodes
+struct PairSplit
+{
+    int groups = 1, parts = 1;
+};
+
+// sum over the LANES neighbouring lanes that share a secondary node
+template <int LANES> __device__ __forceinline__ double laneSum(double v)
+{
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off /= 2)
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
 
 // What a warp needs of its current arrangement and primary, written by lane 0
 // into shared memory and read back by all lanes inside the secondary-node loop
@@ -477,14 +499,6 @@ __device__ __noinline__ double pairA64(const SegmentHeader &h, const double2 *tt
                                        const double2 *pt, double z, double r)
 {
     return segmentA64<1>(h, tt, lt, pt, frameZR(z, r), 0);
-}
-
-__device__ __noinline__ double2 pairB64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                        const double2 *pt, double z, double r)
-{
-    double H, Z;
-    segmentB64<1>(h, tt, lt, pt, frameZR(z, r), 0, H, Z);
-    return make_double2(H, Z);
 }
 
 // The FP32 kernels' FP64 nodes (near-field and refined): FP64 accuracy without
@@ -523,11 +537,6 @@ __device__ __noinline__ double2 pairB32(const SegmentHeader &h, const double2 *t
     return make_double2(H, Z);
 }
 
-// 1: the FP64 kernel calls the out-of-line FP64 quadrature too
-#ifndef CCOIL_PAIR_CALL_FP64
-#define CCOIL_PAIR_CALL_FP64 0
-#endif
-
 // stagedBytes > 0: there is one primary and its whole pair blob (stagedBytes,
 // a multiple of 16) is copied into shared memory once per CTA, so the inner
 // quadrature reads its tables from shared memory instead of through L1.
@@ -547,15 +556,20 @@ __device__ __noinline__ double2 pairB32(const SegmentHeader &h, const double2 *t
 // with the FP64 integrands, 32 at a time like the near-field nodes: the nodes
 // that dominate an arrangement whose ring sum cancels, whose FP32 errors the
 // cancellation magnifies.
-template <int QTY, bool FP32, bool REFINE = false>
-__global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS : CCOIL_PAIR32_MIN_BLOCKS)
-                                               : (QTY == 1 ? CCOIL_PAIR_MIN_BLOCKS_FT : CCOIL_PAIR_MIN_BLOCKS))
+//
+// Few arrangements are cut into more work units than one per arrangement: groups
+// of primaries and, within one primary, ranges of its secondary nodes
+// (PairSplit).  Each unit's sums go to `partial` and pairReduceKernel adds an
+// arrangement's units in a fixed order.  LANES > 1 (FP64 M and F/T): that many
+// lanes share a secondary node and split the primary's angular nodes.
+template <int QTY, bool FP32, bool REFINE = false, int LANES = 1>
+__global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
     pairKernel64(const unsigned char *__restrict__ blob, const long long *__restrict__ primOffsets, int nprim,
                  const double *__restrict__ primPoses, const double *__restrict__ secPoses, long long count,
                  double *__restrict__ out, unsigned long long *__restrict__ zAxisCount, int stagedBytes,
                  const long long *__restrict__ zOffsets, long long *__restrict__ zList,
                  unsigned long long *__restrict__ zListCount, double *__restrict__ nodeScratch, int scratchNodes,
-                 double fraction)
+                 double fraction, PairSplit split, double *__restrict__ partial)
 {
     extern __shared__ __align__(16) unsigned char stagedPair[];
     __shared__ WarpPose warpPoses[4];
@@ -582,13 +596,19 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
     const long long warps = (long long)gridDim.x * blockDim.x / 32;
     double *part = &laneSums[0][threadIdx.x];  // part[128 i]: this thread's sum i
     double *total = warpSums[threadIdx.x / 32];
-    for (long long a = warp; a < count; a += warps)
+    const int perArr = split.groups * split.parts;
+    const long long units = count * perArr;
+    for (long long u = warp; u < units; u += warps)
     {
+        const long long a = u / perArr;
+        const int piece = (int)(u - a * perArr), group = piece / split.parts, part_i = piece - group * split.parts;
+        const int j0 = (int)((long long)nprim * group / split.groups);
+        const int j1 = (int)((long long)nprim * (group + 1) / split.groups);
         if (lane == 0)
             for (int i = 0; i < W; ++i)
                 total[i] = 0.0;
         bool hasZ = false;  // lane 0: some primary of this arrangement is left to the z-axis pass
-        for (int j = 0; j < nprim; ++j)
+        for (int j = j0; j < j1; ++j)
         {
             const unsigned char *base = stagedBytes > 0 ? stagedPair : blob + primOffsets[j];
             const PairHeader &ph = *reinterpret_cast<const PairHeader *>(base);
@@ -629,7 +649,7 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
                     ppose[4] = ph.prim_z_angle;
                 }
                 const bool isZ = zAxisCase(ppose, spose, h.inner_radius);
-                if (zAxisCount && isZ)
+                if (zAxisCount && isZ && part_i == 0)
                     atomicAdd(zAxisCount, 1ull);
                 const bool skip = isZ && zOffsets && zOffsets[j] >= 0;
                 S.skip = skip ? 1 : 0;
@@ -669,7 +689,12 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
             __syncwarp();
             if (S.skip)
                 continue;  // warp-uniform: the z-axis pass adds this primary
-            const int nsec = ph.s_nl * ph.s_nt * ph.s_na;
+            // this unit's secondary nodes: whole warp iterations of 32 / LANES nodes
+            constexpr int STEP = 32 / LANES;
+            const int nodes = ph.s_nl * ph.s_nt * ph.s_na, iters = (nodes + STEP - 1) / STEP;
+            const int nBegin = (int)((long long)iters * part_i / split.parts) * STEP;
+            const int nsec = min(nodes, (int)((long long)iters * (part_i + 1) / split.parts) * STEP);
+            const int sub = lane % LANES, slot = lane / LANES;
             for (int i = 0; i < W; ++i)
                 part[128 * i] = 0.0;
             // every lane runs the same number of iterations (warp-uniform choices
@@ -717,7 +742,7 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
                 {
                     double av;
                     if (!FP32)
-                        av = CCOIL_PAIR_CALL_FP64 ? pairA64(h, tt, lt, pt, f.z, f.r) : segmentA64<1>(h, tt, lt, pt, f, 0);
+                        av = laneSum<LANES>(segmentA64<LANES>(h, tt, lt, pt, f, sub));
                     else if (far)
                         av = pairA32(h, tt, lt, pn, f.z, f.r);
                     else
@@ -846,13 +871,16 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
                 else
                 {
                     double H, Z;
-                    if (!FP32 && !CCOIL_PAIR_CALL_FP64)
-                        segmentB64<1>(h, tt, lt, pt, f, 0, H, Z);
+                    if (!FP32)
+                    {
+                        segmentB64<LANES>(h, tt, lt, pt, f, sub, H, Z);
+                        H = laneSum<LANES>(H);
+                        Z = laneSum<LANES>(Z);
+                    }
                     else
                     {
-                        const double2 hz = !FP32 ? pairB64(h, tt, lt, pt, f.z, f.r)
-                                                 : far ? pairB32(h, tt, lt, pn, f.z, f.r)
-                                                       : pairB64Fast(h, tt, lt, pt, f.z, f.r);
+                        const double2 hz = far ? pairB32(h, tt, lt, pn, f.z, f.r)
+                                               : pairB64Fast(h, tt, lt, pt, f.z, f.r);
                         H = hz.x;
                         Z = hz.y;
                     }
@@ -895,13 +923,13 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
             // directly, without the FP32 pass
             const bool allFp64 = REFINE && !(fraction > 0.0);
             if (!FP32)
-                for (int n0 = 0; n0 < nsec; n0 += 32)
-                    node(n0 + lane < nsec ? n0 + lane : nsec - 1, n0 + lane < nsec, 0);
+                for (int n0 = nBegin; n0 < nsec; n0 += STEP)
+                    node(n0 + slot < nsec ? n0 + slot : nsec - 1, sub == 0 && n0 + slot < nsec, 0);
             else if (allFp64)
-                for (int n0 = 0; n0 < nsec; n0 += 32)
+                for (int n0 = nBegin; n0 < nsec; n0 += 32)
                     node(n0 + lane < nsec ? n0 + lane : nsec - 1, n0 + lane < nsec, 2);
             else
-                for (int n0 = 0; n0 < nsec || nNear > 0;)
+                for (int n0 = nBegin; n0 < nsec || nNear > 0;)
                 {
                     if (nNear >= 32 || n0 >= nsec)
                         fp64Batch();  // deferred near-field nodes
@@ -971,13 +999,93 @@ __global__ void __launch_bounds__(128, FP32 ? (REFINE ? CCOIL_PAIR32R_MIN_BLOCKS
         }
         if (lane == 0)
         {
+            double *dst = partial ? partial + W * u : out + W * a;
 #pragma unroll
             for (int i = 0; i < W; ++i)
-                out[W * a + i] = total[i];
-            if (hasZ)
+                dst[i] = total[i];
+            if (hasZ && !partial)
                 zList[atomicAdd(zListCount, 1ull)] = a;
         }
     }
+}
+
+// Adds the units of each arrangement, one warp per arrangement, and lists the
+// arrangements with a primary left to the z-axis pass.
+template <int W>
+__global__ void __launch_bounds__(128) pairReduceKernel(const double *__restrict__ partial, int perArr,
+                                                        const unsigned char *__restrict__ blob,
+                                                        const long long *__restrict__ primOffsets, int nprim,
+                                                        const double *__restrict__ primPoses,
+                                                        const double *__restrict__ secPoses, long long count,
+                                                        double *__restrict__ out,
+                                                        const long long *__restrict__ zOffsets,
+                                                        long long *__restrict__ zList,
+                                                        unsigned long long *__restrict__ zListCount)
+{
+    const int lane = threadIdx.x % 32;
+    const long long warps = (long long)gridDim.x * blockDim.x / 32;
+    for (long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; a < count; a += warps)
+    {
+        double v[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            v[i] = 0.0;
+        for (int k = lane; k < perArr; k += 32)
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                v[i] += partial[(a * perArr + k) * W + i];
+#pragma unroll
+        for (int off = 16; off > 0; off /= 2)
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                v[i] += __shfl_xor_sync(0xffffffffu, v[i], off);
+        if (lane == 0)
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                out[W * a + i] = v[i];
+        if (!zOffsets)
+            continue;
+        bool z = false;
+        for (int j = lane; j < nprim; j += 32)
+        {
+            const PairHeader &ph = *reinterpret_cast<const PairHeader *>(blob + primOffsets[j]);
+            double own[5] = {ph.prim.position[0], ph.prim.position[1], ph.prim.position[2], ph.prim_y_angle,
+                             ph.prim_z_angle};
+            z = z || (zOffsets[j] >= 0 &&
+                      zAxisCase(primPoses ? primPoses + 5 * a : own, secPoses + 5 * a, ph.prim.inner_radius));
+        }
+        if (__any_sync(0xffffffffu, z) && lane == 0)
+            zList[atomicAdd(zListCount, 1ull)] = a;
+    }
+}
+
+// How `count` arrangements are cut into units for warps of which `resident` run
+// at once.  `nodes`: the largest secondary cloud; `step`: secondary nodes per
+// warp iteration.  One unit per arrangement leaves the last wave nearly empty
+// unless there are several waves of them, and the machine idle below one, so
+// units are made until there are kPairWaves waves: first groups of primaries,
+// then node ranges of equal length (whole iterations) down to one iteration.
+// A unit repeats the arrangement's pose set-up (~2 us of one warp, against
+// 60 us or more for an iteration of M at PrecisionFactor 5).  Whole calls, before
+// and after: one M 745 -> 113 us (with 8 lanes per secondary node; its host work
+// takes ~90 us of both), 1,000 parameter gradients 7.5 -> 4.2 ms, 4,099 M (1.7
+// waves of whole arrangements) 2.72 -> 2.68 ms.
+constexpr long long kPairWaves = 8;
+PairSplit pairSplit(long long count, int nprim, int nodes, int step, long long resident)
+{
+    PairSplit s;
+    const long long want = (kPairWaves * resident + count - 1) / count;  // units per arrangement
+    if (want <= 1)
+        return s;
+    s.groups = (int)std::min<long long>(nprim, want);
+    const int iters = (nodes + step - 1) / step;
+    if (s.groups == nprim && want > nprim)
+    {
+        const long long parts = std::min<long long>((want + nprim - 1) / nprim, iters);
+        const long long each = iters / parts;  // iterations per part, at least
+        s.parts = (int)((iters + each - 1) / each);
+    }
+    return s;
 }
 
 void put(std::vector<unsigned char> &blob, const void *p, size_t n)
@@ -1250,7 +1358,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
             if (!buildZAxis(primaries[j], *secondary, zaxis_precisions[2 * j], zaxis_precisions[2 * j + 1], blob, err))
                 return fail(CCOIL_ERR_INVALID_ARGUMENT, "primary " + std::to_string(j) + ": " + err);
         }
-    DevBuf dBlob, dOff, dPrim, dSec, dOut, dZ, dZOff, dZList, dZCount, dScratch;
+    DevBuf dBlob, dOff, dPrim, dSec, dOut, dZ, dZOff, dZList, dZCount, dScratch, dPartial;
     cudaError_t e = dBlob.alloc(blob.size(), st);
     if (e == cudaSuccess)
         e = dOff.alloc(sizeof(long long) * offsets.size(), st);
@@ -1303,20 +1411,38 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
                              generalBytes % 16 == 0)
                                 ? (int)generalBytes
                                 : 0;
-    const long long warpsNeeded = count;
-    long long blocks = (warpsNeeded + 3) / 4;
+    int secNodes = 0;
+    for (long long off : offsets)
+    {
+        const PairHeader *ph = reinterpret_cast<const PairHeader *>(blob.data() + off);
+        secNodes = std::max(secNodes, ph->s_nl * ph->s_nt * ph->s_na);
+    }
+    // work units (the refining kernel needs a primary's whole total in one warp)
+    const long long resident = 148LL * 4 * pairMinBlocks(quantity, fp32, refine);
+    PairSplit split;
+    int lanes = 1;
+    if (!refine)
+    {
+        // fewer warp iterations in all than resident warps: 8 lanes share a secondary node
+        if (!fp32 && quantity <= CCOIL_PAIR_FORCE_TORQUE && count * primary_count * ((secNodes + 31) / 32) < resident)
+            lanes = 8;
+        split = pairSplit(count, primary_count, secNodes, 32 / lanes, resident);
+    }
+    const long long perArr = (long long)split.groups * split.parts;
+    if (perArr > 1)
+    {
+        e = dPartial.alloc(sizeof(double) * (size_t)width * (size_t)(count * perArr), st);
+        if (e != cudaSuccess)
+            return cudaFail(e, "arrangement partial sums");
+    }
+    long long blocks = (count * perArr + 3) / 4;
     if (blocks > 148LL * 64)
         blocks = 148LL * 64;
     // FP32_REFINED: every warp's region of node contributions (the grid strides over
     // the arrangements, so the scratch is sized by the grid, not by the count)
-    int scratchNodes = 0;
+    const int scratchNodes = refine ? secNodes : 0;
     if (refine)
     {
-        for (long long off : offsets)
-        {
-            const PairHeader *ph = reinterpret_cast<const PairHeader *>(blob.data() + off);
-            scratchNodes = std::max(scratchNodes, ph->s_nl * ph->s_nt * ph->s_na);
-        }
         // at most kPairRefineScratchBytes: a secondary with many nodes runs on fewer
         // warps (each keeps 1 or 6 doubles per node), never fewer than one CTA per SM
         const size_t perBlock = sizeof(double) * (size_t)width * (size_t)scratchNodes * 4;
@@ -1328,6 +1454,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     }
     const double fraction = refineFraction();
     auto *scratch = static_cast<double *>(dScratch.p);
+    auto *partial = static_cast<double *>(dPartial.p);
     auto *zc = static_cast<unsigned long long *>(dZ.p);
     const auto *dB = static_cast<const unsigned char *>(dBlob.p);
     const auto *dO = static_cast<const long long *>(dOff.p);
@@ -1337,8 +1464,13 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     auto *zN = static_cast<unsigned long long *>(dZCount.p);
 #define CCOIL_PAIR_LAUNCH(Q, F, ...)                                                                                   \
     pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, 128, smem, st>>>(                                          \
-        dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction)
-    if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32)
+        dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction,  \
+        split, partial)
+    if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32 && lanes == 8)
+        CCOIL_PAIR_LAUNCH(0, false, false, 8);
+    else if (quantity == CCOIL_PAIR_FORCE_TORQUE && !fp32 && lanes == 8)
+        CCOIL_PAIR_LAUNCH(1, false, false, 8);
+    else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32)
         CCOIL_PAIR_LAUNCH(0, false);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && refine)
         CCOIL_PAIR_LAUNCH(0, true, true);
@@ -1357,6 +1489,22 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     else
         CCOIL_PAIR_LAUNCH(3, true);
 #undef CCOIL_PAIR_LAUNCH
+    if (partial && cudaGetLastError() == cudaSuccess)
+    {
+        const unsigned grid = (unsigned)std::min<long long>((count + 3) / 4, 148LL * 16);
+#define CCOIL_PAIR_REDUCE(W)                                                                                        \
+    pairReduceKernel<W><<<grid, 128, 0, st>>>(partial, (int)perArr, dB, dO, primary_count, primP, secP, count, o,   \
+                                              zPass ? zO : nullptr, zL, zN)
+        if (width == 1)
+            CCOIL_PAIR_REDUCE(1);
+        else if (width == 3)
+            CCOIL_PAIR_REDUCE(3);
+        else if (width == 6)
+            CCOIL_PAIR_REDUCE(6);
+        else
+            CCOIL_PAIR_REDUCE(14);
+#undef CCOIL_PAIR_REDUCE
+    }
     if (zPass && cudaGetLastError() == cudaSuccess)
     {
         // the z-axis pass: one warp per recorded arrangement
