@@ -138,15 +138,52 @@ int DeviceBuffer::reserve(size_t n)
     return CCOIL_OK;
 }
 
-int autoLanes(long long npts)
+// FP32 modes: enough threads to fill the 148 SMs several times over; below that,
+// split the angular nodes of each point across lanes (a lane count is part of an
+// FP32 sum's order, so this rule stands however the work is cut into pieces)
+int autoLanes32(long long npts)
 {
-    // enough threads to fill the 148 SMs several times over; below that, split
-    // the angular nodes of each point across lanes
     const long long target = 148LL * 1024;
     int lanes = 1;
     while (lanes < 8 && npts * lanes < target)
         lanes *= 2;
     return lanes;
+}
+
+// FP64: points and pieces (segments x thickness nodes) fill the machine first,
+// because lanes that share a point repeat every thickness node's set-up (8 lanes
+// and 59 angular nodes: a fifth of the work); lanes come in where those are too
+// few for two waves, and to give the warps of a few points something to do
+int autoLanes64(long long npts, long long pieces, int blocksPerSM)
+{
+    const long long target = 2 * 148LL * 128 * blocksPerSM;
+    int lanes = 1;
+    while (lanes < 32 && npts * lanes * pieces < target)
+        lanes *= 2;
+    return lanes;
+}
+
+// Pieces per tile of points (FieldSplit): the tiles alone leave the last wave
+// nearly empty unless there are several waves of them, and the machine idle below
+// one, so segments are dealt out, and then every segment's thickness nodes, until
+// there are kFieldWaves waves of blocks.  A piece repeats its points' frame
+// transform, so beyond one wave it keeps kPieceNodes nodes per thread.  FP64 kernel
+// times before and after: A of 24 coils at 1,001 points 310 -> 93 us, B of 64 coils
+// at 4,096 points 1.73 -> 1.07 ms, B of one coil at 37 points 24 -> 8 us; FP32_REFINED
+// A of 128 coils at 200,003 points (2.1 waves whole) 20.4 -> 18.5 ms.
+constexpr long long kFieldWaves = 8, kPieceNodes = 128;
+FieldSplit fieldSplit(long long npts, int lanes, int nseg, int thickness, long long nodes, int blocksPerSM,
+                      bool wholeSegments)
+{
+    FieldSplit s;
+    const long long wave = 148LL * blocksPerSM;
+    const long long tiles = (npts + 128 / lanes - 1) / (128 / lanes);
+    const long long one = (wave + tiles - 1) / tiles, full = (kFieldWaves * wave + tiles - 1) / tiles;
+    const long long want = std::min(full, std::max(one, nodes / (lanes * kPieceNodes)));
+    s.groups = (int)std::max(1LL, std::min<long long>(want, nseg));
+    if (s.groups == nseg && !wholeSegments)
+        s.parts = (int)std::max(1LL, std::min<long long>((want + nseg - 1) / nseg, thickness));
+    return s;
 }
 
 bool validLanes(int l) { return l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32; }
@@ -160,6 +197,8 @@ struct ccoil_field_plan
     int field = 0;
     int precision = 0;
     int coil_count = 0;
+    int thickness = 1;    // most thickness nodes of a segment
+    long long nodes = 0;  // quadrature nodes of all segments
     SegmentSet set;
     DeviceBuffer blob, segs, points, out, work, workCount;
     DeviceBuffer contrib, refineSegs, refinedTotal;  // FP32_REFINED
@@ -249,6 +288,12 @@ int ccoil_field_plan_create(const ccoil_coil_t *coils, int coil_count, int field
         delete p;
         return fail(CCOIL_ERR_INVALID_ARGUMENT, err);
     }
+    for (const SegmentDesc &d : p->set.segs)
+    {
+        const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(p->set.blob.data() + d.offset);
+        p->thickness = std::max(p->thickness, h.n_t);
+        p->nodes += (long long)h.n_t * h.n_phi * std::max(h.n_l, 1);
+    }
     if (!p->set.segs.empty())
     {
         int rc = p->blob.reserve(p->set.blob.size());
@@ -320,7 +365,10 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
     L.d_out = dOut;
     L.field = plan->field;
     L.precision = plan->precision;
-    L.lanes = lanes_per_point ? lanes_per_point : autoLanes(point_count);
+    const int perSM = fieldBlocksPerSM(plan->field, plan->precision);
+    L.lanes = lanes_per_point                              ? lanes_per_point
+              : plan->precision == CCOIL_PRECISION_FP64 ? autoLanes64(point_count, (long long)L.nseg * plan->thickness, perSM)
+                                                        : autoLanes32(point_count);
     // FP32_REFINED runs in chunks of points whose stored contributions fit
     // kRefineContribBytes and whose pairs fit a list of kRefineListPairs
     const bool refined = plan->precision == CCOIL_PRECISION_FP32_REFINED && L.nseg > 0;
@@ -396,6 +444,29 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
         L.d_points = static_cast<const double *>(plan->sortedPoints.ptr);
         L.d_out = static_cast<double *>(plan->sortedOut.ptr);
     }
+    // the pieces' sums: memory of this call alone (a plan may run on several streams
+    // at once), in the order of the stream.  Without it, or while the stream is
+    // captured (a captured call must not hold an allocation that each replay would
+    // make again), the points are evaluated in one piece
+    void *partial = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (L.nseg > 0 && perSM > 0 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone)
+    {
+        const FieldSplit split = fieldSplit(chunk, L.lanes, L.nseg, plan->thickness, plan->nodes, perSM,
+                                            refined);
+        const size_t pieces = (size_t)split.groups * (size_t)split.parts;
+        if (pieces > 1 && scratchAlloc(&partial, pieces * (size_t)chunk * width * sizeof(double), st) == cudaSuccess)
+        {
+            L.split = split;
+            L.d_partial = static_cast<double *>(partial);
+        }
+        else
+        {
+            partial = nullptr;
+            cudaGetLastError();  // an allocation that failed is not this call's error
+        }
+    }
     int rc = CCOIL_OK;
     for (long long off = 0; off < point_count && rc == CCOIL_OK; off += chunk)
     {
@@ -405,6 +476,8 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
         C.npts = std::min(chunk, point_count - off);
         rc = launchFields(C, stream);
     }
+    if (partial)
+        cudaFreeAsync(partial, st);
     if (rc == CCOIL_OK && ordered)
         rc = scatterResults(static_cast<const double *>(plan->sortedOut.ptr), static_cast<const int *>(plan->order.ptr),
                             point_count, width, dOut, stream);

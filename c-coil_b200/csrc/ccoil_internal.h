@@ -158,6 +158,14 @@ int failMessage(int status, const char *msg);  // same, without building a std::
 // scratchAlloc/cudaFreeAsync are ordered on `st`.
 cudaError_t scratchAlloc(void **p, size_t bytes, cudaStream_t st);
 
+// How a field evaluation is cut into pieces beyond its points: `groups` of
+// segments times `parts` of every segment's thickness nodes.  More than one piece
+// needs d_partial (pieces x points x W doubles), which is summed in order.
+struct FieldSplit
+{
+    int groups = 1, parts = 1;
+};
+
 // kernels (fields.cu)
 struct FieldLaunch
 {
@@ -175,6 +183,8 @@ struct FieldLaunch
     unsigned long long work_capacity = 0;
     unsigned long long *d_work_count = nullptr;
     int near_blocks = 0;                    // grid of the near-field pass
+    FieldSplit split;
+    double *d_partial = nullptr;
     // FP32_REFINED: every (point, segment) FP32 contribution whose norm exceeds
     // refine_fraction times the norm of the point's total is replaced by its
     // FP64 value; the FP32 pass stores the contributions in d_contrib
@@ -199,6 +209,8 @@ double refineFraction();  // the process-wide fraction (ccoil_set_refine_fractio
 constexpr size_t kRefineContribBytes = size_t(1) << 32;
 constexpr unsigned long long kRefineListPairs = 1ULL << 28;
 int launchFields(const FieldLaunch &L, void *stream);
+// CTAs of 128 threads that one SM holds of the kernel for (field, precision)
+int fieldBlocksPerSM(int field, int precision);
 int readTimeouts(long long &count);
 
 // Point ordering of the FP32 field plans (ordering.cu): sort the points along

@@ -138,7 +138,8 @@ template <int FIELD, int LANES>
 __global__ void __launch_bounds__(128, fp64MinBlocks(FIELD)) fieldsKernel64(const unsigned char *__restrict__ blob,
                                                       const SegmentDesc *__restrict__ segs, int nseg,
                                                       const double *__restrict__ points, long long npts,
-                                                      double *__restrict__ out)
+                                                      double *__restrict__ out, FieldSplit split,
+                                                      double *__restrict__ partial)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -172,11 +173,16 @@ __global__ void __launch_bounds__(128, fp64MinBlocks(FIELD)) fieldsKernel64(cons
     for (int i = 0; i < W; ++i)
         acc[i] = 0.0;
 
-    for (int s = 0; s < nseg; ++s)
+    // this block's piece of the work (FieldSplit)
+    const int piece = blockIdx.y, group = piece / split.parts;
+    const Slice th = {piece - group * split.parts, split.parts};
+    const int sBegin = (int)((long long)nseg * group / split.groups);
+    const int sEnd = (int)((long long)nseg * (group + 1) / split.groups);
+    for (int s = sBegin; s < sEnd; ++s)
     {
 #if !CCOIL_FP64_STAGE
         if (active)
-            integrateSegment64<FIELD, LANES>(blob + segs[s].offset, px, py, pz, lane, acc);
+            integrateSegment64<FIELD, LANES>(blob + segs[s].offset, px, py, pz, lane, acc, th);
 #else
         const int stage = s % kSegmentStages;
         const unsigned parity = (unsigned)((s / kSegmentStages) & 1);
@@ -216,9 +222,39 @@ __global__ void __launch_bounds__(128, fp64MinBlocks(FIELD)) fieldsKernel64(cons
             acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
     if (active && lane == 0)
     {
+        double *dst = partial ? partial + ((size_t)piece * (size_t)npts + (size_t)p) * W : out + W * p;
 #pragma unroll
         for (int i = 0; i < W; ++i)
-            out[W * p + i] = acc[i];
+            dst[i] = acc[i];
+    }
+}
+
+// out[i] = the sum of the pieces' values i.  A block takes 32 values; its ROWS
+// rows of 32 threads take every ROWS-th piece each and are added in order, so the
+// result repeats exactly and a few values of many pieces are not one long chain
+// of loads.
+template <int ROWS>
+__global__ void __launch_bounds__(32 * ROWS) sumPiecesKernel(const double *__restrict__ partial, int pieces,
+                                                             long long n, double *__restrict__ out)
+{
+    __shared__ double rows[ROWS][32];
+    const int x = threadIdx.x % 32, y = threadIdx.x / 32;
+    const long long i = (long long)blockIdx.x * 32 + x;
+    double v = 0.0;
+    if (i < n)
+    {
+#pragma unroll 4
+        for (int k = y; k < pieces; k += ROWS)
+            v += partial[(long long)k * n + i];
+    }
+    rows[y][x] = v;
+    __syncthreads();
+    if (y == 0 && i < n)
+    {
+#pragma unroll
+        for (int r = 1; r < ROWS; ++r)
+            v += rows[r][x];
+        out[i] = v;
     }
 }
 
@@ -242,12 +278,17 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
     const bool staged = fp32 ? CCOIL_FP32_STAGE : CCOIL_FP64_STAGE;
     const size_t smem = staged ? (size_t)kSegmentStages * kSegmentBytes : 0;
     NearPair *work = reinterpret_cast<NearPair *>(L.d_work);
+    const int pieces = L.split.groups * L.split.parts;
+    if ((pieces > 1 && (!L.d_partial || staged)) || pieces > 65535 || (refine && L.split.parts > 1))
+        return cudaErrorInvalidValue;
+    double *partial = pieces > 1 ? L.d_partial : nullptr;
+    const dim3 grid((unsigned)blocks, (unsigned)pieces);
     switch (L.lanes)
     {
 #define CCOIL_LAUNCH32(N, R)                                                                                      \
-    fieldsKernel32<FIELD, N, R><<<(unsigned)blocks, threads, smem, st>>>(                                         \
-        L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, L.d_out, work, L.work_capacity, L.d_work_count,           \
-        R ? L.d_contrib : nullptr)
+    fieldsKernel32<FIELD, N, R><<<grid, threads, smem, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts,     \
+                                                             L.d_out, work, L.work_capacity, L.d_work_count,      \
+                                                             R ? L.d_contrib : nullptr, L.split, partial)
 #define CCOIL_CASE(N, REFINING)                                                                                   \
     case N:                                                                                                       \
         if (refine)                                                                                               \
@@ -255,8 +296,8 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
         else if (fp32)                                                                                            \
             CCOIL_LAUNCH32(N, false);                                                                             \
         else                                                                                                      \
-            fieldsKernel64<FIELD, N><<<(unsigned)blocks, threads, smem, st>>>(L.d_blob, L.d_segs, L.nseg,         \
-                                                                              L.d_points, L.npts, L.d_out);       \
+            fieldsKernel64<FIELD, N><<<grid, threads, smem, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, \
+                                                                  L.d_out, L.split, partial);                     \
         break;
         CCOIL_CASE(1, true)
         CCOIL_CASE(2, true)
@@ -269,6 +310,15 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
         default: return cudaErrorInvalidValue;
     }
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && partial)
+    {
+        const long long n = L.npts * (FIELD == CCOIL_FIELD_G ? 9 : 3);
+        if (pieces <= 64)
+            sumPiecesKernel<4><<<(unsigned)((n + 31) / 32), 128, 0, st>>>(partial, pieces, n, L.d_out);
+        else
+            sumPiecesKernel<32><<<(unsigned)((n + 31) / 32), 1024, 0, st>>>(partial, pieces, n, L.d_out);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess || !fp32)
         return e;
     // near-field pairs in FP64; the grid loops over the device-side count, so no
@@ -332,6 +382,13 @@ int launchFields(const FieldLaunch &L, void *stream)
     if (e != cudaSuccess)
         return failMessage(CCOIL_ERR_CUDA, cudaGetErrorString(e));
     return CCOIL_OK;
+}
+
+int fieldBlocksPerSM(int field, int precision)
+{
+    if (precision == CCOIL_PRECISION_FP64)
+        return CCOIL_FP64_STAGE ? 0 : fp64MinBlocks(field);
+    return CCOIL_FP32_STAGE ? 0 : fp32MinBlocks(field);
 }
 
 int launchBatch(const BatchLaunch &B, void *stream)

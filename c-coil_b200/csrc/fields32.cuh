@@ -20,7 +20,8 @@
 
 // Integrates one segment for one lane and adds the lane's contribution to acc.
 template <int FIELD, int LANES>
-__device__ __forceinline__ void integrateSegment32(const unsigned char *seg, const Frame &f, int lane, double *acc)
+__device__ __forceinline__ void integrateSegment32(const unsigned char *seg, const Frame &f, int lane, double *acc,
+                                                   Slice th = Slice())
 {
     const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
     const double2 *tt = reinterpret_cast<const double2 *>(seg) + h.off_t;
@@ -29,18 +30,18 @@ __device__ __forceinline__ void integrateSegment32(const unsigned char *seg, con
     if (FIELD == CCOIL_FIELD_B)
     {
         double H, Z;
-        segmentB32<LANES>(h, tt, lt, pn, f, lane, H, Z);
+        segmentB32<LANES>(h, tt, lt, pn, f, lane, H, Z, th);
         addRotated(h, H * f.cphi, H * f.sphi, Z, acc);
     }
     else if (FIELD == CCOIL_FIELD_G)
     {
         double g[4];
-        segmentG32<LANES>(h, tt, lt, pn, f, lane, g);
+        segmentG32<LANES>(h, tt, lt, pn, f, lane, g, th);
         addGradient(h, f, g, acc);
     }
     else
     {
-        double a = segmentA32<LANES>(h, tt, lt, pn, f, lane) * h.field_factor;
+        double a = segmentA32<LANES>(h, tt, lt, pn, f, lane, th) * h.field_factor;
         addRotated(h, -a * f.sphi, a * f.cphi, 0.0, acc);
     }
 }
@@ -98,7 +99,8 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
                                                       double *__restrict__ out, NearPair *__restrict__ work,
                                                       unsigned long long workCapacity,
                                                       unsigned long long *__restrict__ workCount,
-                                                      double *__restrict__ contrib)
+                                                      double *__restrict__ contrib, FieldSplit split,
+                                                      double *__restrict__ partial)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -133,12 +135,17 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
 #pragma unroll
     for (int i = 0; i < W; ++i)
         acc[i] = 0.0;
+    // this block's piece of the work (FieldSplit)
+    const int piece = blockIdx.y, group = piece / split.parts;
+    const Slice th = {piece - group * split.parts, split.parts};
+    const int sBegin = (int)((long long)nseg * group / split.groups);
+    const int sEnd = (int)((long long)nseg * (group + 1) / split.groups);
     // the lanes of one point
     auto groupMask = [] {
         return LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << ((threadIdx.x % 32) / LANES * LANES));
     };
 
-    for (int s = 0; s < nseg; ++s)
+    for (int s = sBegin; s < sEnd; ++s)
     {
 #if CCOIL_FP32_STAGE
         const int stage = s % kSegmentStages;
@@ -157,7 +164,9 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
             const Frame f = toCoilFrame(h, px, py, pz);
             const bool nearPair = nearWinding(h, f);
             if (!nearPair && !REFINE)
-                integrateSegment32<FIELD, LANES>(seg, f, lane, acc);
+                integrateSegment32<FIELD, LANES>(seg, f, lane, acc, th);
+            else if (nearPair && th.i != 0)
+                continue;  // the first part lists the pair
             else if (!nearPair)
             {
                 // the segment's contribution on its own: combined over the point's
@@ -241,9 +250,10 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
             acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
     if (active && lane == 0)
     {
+        double *dst = partial ? partial + ((size_t)piece * (size_t)npts + (size_t)p) * W : out + W * p;
 #pragma unroll
         for (int i = 0; i < W; ++i)
-            out[W * p + i] = acc[i];
+            dst[i] = acc[i];
     }
 }
 

@@ -368,7 +368,8 @@ __device__ __forceinline__ PairInv pairInverse(V2 a, V2 b)
 // UNIFORM: warp-uniform slab branches (bySlab)
 template <int LANES, typename S = F64Sum, bool UNIFORM = true>
 __device__ __forceinline__ double segmentA32(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                             const PhiPair2 *pn, const Frame &f, int lane)
+                                             const PhiPair2 *pn, const Frame &f, int lane,
+                                             Slice th = Slice())
 {
     double sum = 0.0;
     const int ne = packedEntries(h.n_phi);
@@ -382,7 +383,7 @@ __device__ __forceinline__ double segmentA32(const SegmentHeader &h, const doubl
         const V2 TOP = v2(topf), BOT = v2(botf), NBOT = v2(-botf), DDF = v2(dDf), DDL = v2(dDl);
         bySlab<UNIFORM>(same, [&](auto slab) {
             const bool outside = slabOutside<decltype(slab)::value>(same);
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double q = (t.x - f.r) * (t.x - f.r), b2d = 2.0 * t.x * f.r;
@@ -459,7 +460,7 @@ __device__ __forceinline__ double segmentA32(const SegmentHeader &h, const doubl
         {
             const double2 l = lt[i];
             const double zl = l.x + f.z;
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double q = (t.x - f.r) * (t.x - f.r) + zl * zl, b2d = 2.0 * t.x * f.r;
@@ -496,7 +497,8 @@ __device__ __forceinline__ double segmentA32(const SegmentHeader &h, const doubl
 //   H: w c (g^3 - g'^3) = b2 w2c2 k3,   Z: w (2 p^2 g'^3 + num delta k3).
 template <int LANES, typename S = F64Sum, bool UNIFORM = true>
 __device__ __forceinline__ void segmentB32(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                           const PhiPair2 *pn, const Frame &f, int lane, double &H, double &Z)
+                                           const PhiPair2 *pn, const Frame &f, int lane, double &H, double &Z,
+                                           Slice th = Slice())
 {
     H = 0.0;
     Z = 0.0;
@@ -511,7 +513,7 @@ __device__ __forceinline__ void segmentB32(const SegmentHeader &h, const double2
         bySlab<UNIFORM>(same, [&](auto slab) {
             const bool outside = slabOutside<decltype(slab)::value>(same);
             const double zScale = outside ? dD : 1.0;
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double q = (t.x - f.r) * (t.x - f.r), b2d = 2.0 * t.x * f.r;
@@ -565,7 +567,7 @@ __device__ __forceinline__ void segmentB32(const SegmentHeader &h, const double2
         {
             const double2 l = lt[i];
             const double zl = l.x + f.z;
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double q = (t.x - f.r) * (t.x - f.r) + zl * zl, b2d = 2.0 * t.x * f.r;
@@ -745,7 +747,8 @@ __device__ __forceinline__ void segmentB32Direct(const SegmentHeader &h, const d
 // {RPhi, RR, RZ, ZZ}
 template <int LANES>
 __device__ __forceinline__ void segmentG32(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                           const PhiPair2 *pn, const Frame &f, int lane, double *g)
+                                           const PhiPair2 *pn, const Frame &f, int lane, double *g,
+                                           Slice th = Slice())
 {
     double rphi = 0.0, rr = 0.0, rz = 0.0, zz = 0.0;
     const double r = f.r;
@@ -784,7 +787,7 @@ __device__ __forceinline__ void segmentG32(const SegmentHeader &h, const double2
                 cz = T1 + Y;
                 kz = fma2(v2(2.0f), Y, T1) * rrho;
             };
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double q = (t.x - r) * (t.x - r), b2d = 2.0 * t.x * r;
@@ -819,7 +822,7 @@ __device__ __forceinline__ void segmentG32(const SegmentHeader &h, const double2
         {
             const double2 l = lt[i];
             const double zl = l.x + f.z;
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double p = t.x;

@@ -17,6 +17,14 @@
 // fp64ops.cuh were cut further, the last two)
 constexpr int kUnroll64 = 4;
 
+// part i of n of a segment's thickness nodes (the field kernels split few points
+// this way); the default is all of them
+struct Slice
+{
+    int i = 0, n = 1;
+    __device__ __forceinline__ int begin(int nodes) const { return nodes * i / n; }
+    __device__ __forceinline__ int end(int nodes) const { return nodes * (i + 1) / n; }
+};
 
 struct Frame
 {
@@ -109,7 +117,8 @@ __device__ __noinline__ double phiSlowA64Ieee(const double2 *pt, int n, int lane
 
 template <int LANES>
 __device__ __forceinline__ double segmentA64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                             const double2 *pt, const Frame &f, int lane)
+                                             const double2 *pt, const Frame &f, int lane,
+                                             Slice th = Slice())
 {
     double sum = 0.0;
     const int n = h.n_phi;
@@ -118,7 +127,7 @@ __device__ __forceinline__ double segmentA64(const SegmentHeader &h, const doubl
         // CalculateFieldsFast.cxx:27-78
         const double top = add(f.z, h.half_length), bot = sub(f.z, h.half_length);
         const double far2 = fmax(top * top, bot * bot);
-        for (int j = 0; j < h.n_t; ++j)
+        for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
         {
             const double2 t = tt[j];
             const double cA = mul(mul(2.0, t.x), f.r);
@@ -149,7 +158,7 @@ __device__ __forceinline__ double segmentA64(const SegmentHeader &h, const doubl
         {
             const double2 l = lt[i];
             const double zl = add(l.x, f.z);
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double cA = mul(mul(2.0, t.x), f.r);
@@ -205,7 +214,8 @@ __device__ __noinline__ double2 phiSlowB64Ieee(const double2 *pt, int n, int lan
 
 template <int LANES>
 __device__ __forceinline__ void segmentB64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                           const double2 *pt, const Frame &f, int lane, double &H, double &Z)
+                                           const double2 *pt, const Frame &f, int lane, double &H, double &Z,
+                                           Slice th = Slice())
 {
     H = 0.0;
     Z = 0.0;
@@ -214,7 +224,7 @@ __device__ __forceinline__ void segmentB64(const SegmentHeader &h, const double2
     {
         // CalculateFieldsFast.cxx:100-155
         const double top = add(f.z, h.half_length), bot = sub(f.z, h.half_length);
-        for (int j = 0; j < h.n_t; ++j)
+        for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
         {
             const double2 t = tt[j];
             const double cA = mul(t.x, t.x), cB = mul(t.x, f.r);
@@ -251,7 +261,7 @@ __device__ __forceinline__ void segmentB64(const SegmentHeader &h, const double2
         {
             const double2 l = lt[i];
             const double zl = add(l.x, f.z);
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double cA = mul(t.x, t.x), cB = mul(t.x, zl), cC = mul(t.x, f.r);
@@ -343,7 +353,8 @@ __device__ __noinline__ double4 phiSlowG64Ieee(const double2 *pt, int n, int lan
 // {RPhi, RR, RZ, ZZ}
 template <int LANES>
 __device__ __forceinline__ void segmentG64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                           const double2 *pt, const Frame &f, int lane, double *g)
+                                           const double2 *pt, const Frame &f, int lane, double *g,
+                                           Slice th = Slice())
 {
     double rphi = 0.0, rr = 0.0, rz = 0.0, zz = 0.0;
     const double r = f.r;
@@ -355,7 +366,7 @@ __device__ __forceinline__ void segmentG64(const SegmentHeader &h, const double2
         // they are all that is left of it.  What only scales a node's term
         // (p c / r, w p / M^2) is rounded on its own
         const double top = add(f.z, h.half_length), bot = sub(f.z, h.half_length);
-        for (int j = 0; j < h.n_t; ++j)
+        for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
         {
             const double2 t = tt[j];
             const double A = mul(t.x, t.x), B = mul(r, r), C = mul(t.x, r);
@@ -411,7 +422,7 @@ __device__ __forceinline__ void segmentG64(const SegmentHeader &h, const double2
         {
             const double2 l = lt[i];
             const double zl = add(l.x, f.z);
-            for (int j = 0; j < h.n_t; ++j)
+            for (int j = th.begin(h.n_t), jEnd = th.end(h.n_t); j < jEnd; ++j)
             {
                 const double2 t = tt[j];
                 const double A = mul(t.x, t.x), B = mul(r, r), C = mul(zl, zl);
@@ -506,28 +517,30 @@ __device__ __forceinline__ void addGradient(const SegmentHeader &h, const Frame 
 
 template <int FIELD, int LANES>
 __device__ __forceinline__ void integrateSegment64(const unsigned char *seg, double px, double py, double pz, int lane,
-                                                   double *acc)
+                                                   double *acc, Slice th = Slice())
 {
     const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
     const double2 *tt = reinterpret_cast<const double2 *>(seg) + h.off_t;
     const double2 *lt = reinterpret_cast<const double2 *>(seg) + h.off_l;
     const double2 *pt = reinterpret_cast<const double2 *>(seg) + h.off_phi;
+    if (th.begin(h.n_t) == th.end(h.n_t))
+        return;  // fewer thickness nodes than parts
     Frame f = toCoilFrame(h, px, py, pz);
     if (FIELD == CCOIL_FIELD_B)
     {
         double H, Z;
-        segmentB64<LANES>(h, tt, lt, pt, f, lane, H, Z);
+        segmentB64<LANES>(h, tt, lt, pt, f, lane, H, Z, th);
         addRotated(h, H * f.cphi, H * f.sphi, Z, acc);
     }
     else if (FIELD == CCOIL_FIELD_G)
     {
         double g[4];
-        segmentG64<LANES>(h, tt, lt, pt, f, lane, g);
+        segmentG64<LANES>(h, tt, lt, pt, f, lane, g, th);
         addGradient(h, f, g, acc);
     }
     else
     {
-        double a = segmentA64<LANES>(h, tt, lt, pt, f, lane) * h.field_factor;
+        double a = segmentA64<LANES>(h, tt, lt, pt, f, lane, th) * h.field_factor;
         addRotated(h, -a * f.sphi, a * f.cphi, 0.0, acc);
     }
 }

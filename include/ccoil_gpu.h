@@ -376,7 +376,8 @@ int ccoil_inject_allocation_failures(int count);
  * allocation.
  * Same arguments as ccoil_compute_fields with precision FP32_COMPENSATED,
  * except that `points` and `out` must be device pointers and the call is
- * asynchronous on `stream`; the same results up to 16,383 points (from 16,384
+ * asynchronous on `stream`; the same results up to the order of FP64 sums up to
+ * 16,383 points (ccoil_compute_fields adds groups of segments; from 16,384
  * on, ccoil_compute_fields evaluates the points in Morton order, see
  * ccoil_set_point_ordering, and the two differ by FP32 rounding; this entry
  * point keeps the caller's order).
