@@ -287,8 +287,7 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
     {
 #define CCOIL_LAUNCH32(N, R)                                                                                      \
     fieldsKernel32<FIELD, N, R><<<grid, threads, smem, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts,     \
-                                                             L.d_out, work, L.work_capacity, L.d_work_count,      \
-                                                             R ? L.d_contrib : nullptr, L.split, partial)
+                                                             L.d_out, R ? L.d_contrib : nullptr, L.split, partial)
 #define CCOIL_CASE(N, REFINING)                                                                                   \
     case N:                                                                                                       \
         if (refine)                                                                                               \
@@ -323,8 +322,10 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
         return e;
     // near-field pairs in FP64; the grid loops over the device-side count, so no
     // host synchronisation is needed between the passes
-    nearFieldKernel<FIELD><<<L.near_blocks, 256, 0, st>>>(L.d_blob, L.d_segs, L.d_points, L.d_out, work,
-                                                            L.work_capacity, L.d_work_count);
+    nearListKernel<<<(unsigned)((L.npts + 255) / 256), 256, 0, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts,
+                                                                     work, L.work_capacity, L.d_work_count);
+    nearFieldKernel<FIELD><<<L.near_blocks, 256, 0, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, L.d_out,
+                                                          work, L.work_capacity, L.d_work_count);
     e = cudaGetLastError();
     if (e != cudaSuccess || !refine)
         return e;

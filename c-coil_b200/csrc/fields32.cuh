@@ -3,10 +3,12 @@
 // the integrands themselves are in integrands32.cuh.
 //
 // Near field.  A point inside a coil's winding box (inflated by a margin) is
-// not integrated by the FP32 loop: its (point, segment) pair goes to a work
-// list and a second kernel evaluates it with the FP64 integrands, so warps
-// never diverge between the two paths.  If the list is full the pair is
-// integrated in FP64 in place.
+// left out by the FP32 loop.  A second kernel lists such (point, segment) pairs,
+// a point's pairs next to each other and in segment order, and a third evaluates
+// them with the FP64 integrands, so warps never diverge between the two paths.
+// One warp adds all pairs of a point, in order: results repeat exactly however the
+// FP32 pass is cut into pieces.  If the list is too short for all pairs, the third
+// kernel finds and evaluates them itself.
 //
 // FP32_REFINED.  The FP32 kernel also stores every (point, segment)
 // contribution; once the point's total is known, a selection kernel removes
@@ -96,10 +98,8 @@ template <int FIELD, int LANES, bool REFINE>
 __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(const unsigned char *__restrict__ blob,
                                                       const SegmentDesc *__restrict__ segs, int nseg,
                                                       const double *__restrict__ points, long long npts,
-                                                      double *__restrict__ out, NearPair *__restrict__ work,
-                                                      unsigned long long workCapacity,
-                                                      unsigned long long *__restrict__ workCount,
-                                                      double *__restrict__ contrib, FieldSplit split,
+                                                      double *__restrict__ out, double *__restrict__ contrib,
+                                                      FieldSplit split,
                                                       double *__restrict__ partial)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
@@ -131,10 +131,19 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
         py = points[3 * p + 1];
         pz = points[3 * p + 2];
     }
+    // the gradient's nine sums live in shared memory, one column per thread: in
+    // registers they spill others at 128 (G of 128 coils at 2^17 points: 17.1 ms
+    // against 19.0)
+    constexpr bool kShared = FIELD == CCOIL_FIELD_G;
+    __shared__ double sums[kShared ? W : 1][128];
     double acc[W];
 #pragma unroll
     for (int i = 0; i < W; ++i)
+    {
         acc[i] = 0.0;
+        if (kShared)
+            sums[kShared ? i : 0][threadIdx.x] = 0.0;
+    }
     // this block's piece of the work (FieldSplit)
     const int piece = blockIdx.y, group = piece / split.parts;
     const Slice th = {piece - group * split.parts, split.parts};
@@ -163,10 +172,19 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
             const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
             const Frame f = toCoilFrame(h, px, py, pz);
             const bool nearPair = nearWinding(h, f);
-            if (!nearPair && !REFINE)
+            if (!nearPair && kShared && !REFINE)
+            {
+                double c[W];
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    c[i] = 0.0;
+                integrateSegment32<FIELD, LANES>(seg, f, lane, c, th);
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    sums[kShared ? i : 0][threadIdx.x] += c[i];
+            }
+            else if (!nearPair && !REFINE)
                 integrateSegment32<FIELD, LANES>(seg, f, lane, acc, th);
-            else if (nearPair && th.i != 0)
-                continue;  // the first part lists the pair
             else if (!nearPair)
             {
                 // the segment's contribution on its own: combined over the point's
@@ -188,35 +206,20 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
 #pragma unroll
                     for (int i = 0; i < W; ++i)
                     {
-                        acc[i] += c[i];
+                        if (kShared)
+                            sums[kShared ? i : 0][threadIdx.x] += c[i];
+                        else
+                            acc[i] += c[i];
                         dst[i] = c[i];
                     }
                 }
             }
-            else
+            else if (REFINE && lane == 0)
             {
-                if (REFINE && lane == 0)
-                {
-                    double *dst = contrib + ((size_t)s * (size_t)npts + (size_t)p) * W;
+                double *dst = contrib + ((size_t)s * (size_t)npts + (size_t)p) * W;
 #pragma unroll
-                    for (int i = 0; i < W; ++i)
-                        dst[i] = 0.0;
-                }
-                bool queued = false;
-                if (lane == 0)
-                {
-                    unsigned long long slot = atomicAdd(workCount, 1ull);
-                    if (slot < workCapacity)
-                    {
-                        work[slot].point = (int)p;
-                        work[slot].segment = s;
-                        queued = true;
-                    }
-                }
-                // all lanes of the point learn whether the pair was queued
-                queued = __shfl_sync(groupMask(), queued, (threadIdx.x % 32) / LANES * LANES);
-                if (!queued)
-                    integrateSegment64Fallback<FIELD, LANES>(seg, px, py, pz, lane, acc);
+                for (int i = 0; i < W; ++i)
+                    dst[i] = 0.0;
             }
         }
 #if CCOIL_FP32_STAGE
@@ -243,6 +246,10 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
 #endif
     }
 
+    if (kShared)
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            acc[i] = sums[kShared ? i : 0][threadIdx.x];
 #pragma unroll
     for (int off = LANES / 2; off > 0; off /= 2)
 #pragma unroll
@@ -257,32 +264,90 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
     }
 }
 
-// Second pass: one warp per near-field (point, segment) pair, FP64 integrands
-// read from the segment blob in global memory, result added to the point's
-// output (FP64 atomics; each pair adds once).
+// whether a point lies in a segment's near box
+__device__ __forceinline__ bool isNearPair(const unsigned char *blob, const SegmentDesc *segs, int s, double px,
+                                           double py, double pz)
+{
+    const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(blob + segs[s].offset);
+    return nearWinding(h, toCoilFrame(h, px, py, pz));
+}
+
+// Lists the near-field pairs, one thread per point: the pairs of a point in one
+// run of entries, in segment order.  It takes every frame transform once more.
+__global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__restrict__ blob,
+                                                         const SegmentDesc *__restrict__ segs, int nseg,
+                                                         const double *__restrict__ points, long long npts,
+                                                         NearPair *__restrict__ work,
+                                                         unsigned long long workCapacity,
+                                                         unsigned long long *__restrict__ workCount)
+{
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npts)
+        return;
+    const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
+    int count = 0, first = nseg;
+#pragma unroll 2
+    for (int s = 0; s < nseg; ++s)
+        if (isNearPair(blob, segs, s, px, py, pz))
+        {
+            first = count == 0 ? s : first;
+            ++count;
+        }
+    if (count == 0)
+        return;
+    unsigned long long slot = atomicAdd(workCount, (unsigned long long)count);
+    for (int s = first; s < nseg && slot < workCapacity; ++s)
+        if (isNearPair(blob, segs, s, px, py, pz))
+        {
+            work[slot].point = (int)p;
+            work[slot].segment = s;
+            ++slot;
+        }
+}
+
+// Evaluates the near-field pairs: one warp per point's run of entries, the FP64
+// integrands read from the segment blob in global memory, the lanes splitting the
+// angular nodes; the warp alone adds to the point's output.  With more pairs than
+// the list holds, the warps go over all points instead.
 template <int FIELD>
 __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__restrict__ blob,
-                                                       const SegmentDesc *__restrict__ segs,
-                                                       const double *__restrict__ points, double *__restrict__ out,
-                                                       const NearPair *__restrict__ work,
+                                                       const SegmentDesc *__restrict__ segs, int nseg,
+                                                       const double *__restrict__ points, long long npts,
+                                                       double *__restrict__ out, const NearPair *__restrict__ work,
                                                        unsigned long long workCapacity,
                                                        const unsigned long long *__restrict__ workCount)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
-    const unsigned long long n = min(*workCount, workCapacity);
+    const unsigned long long n = *workCount;
+    const bool listed = n <= workCapacity;
     const int lane = threadIdx.x % 32;
     const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const unsigned long long warps = (unsigned long long)gridDim.x * blockDim.x / 32;
-    for (unsigned long long i = warp; i < n; i += warps)
+    // entry (listed) or point i; a point's entries are consecutive
+    const unsigned long long end = listed ? n : (unsigned long long)npts;
+    for (unsigned long long i = warp; i < end; i += warps)
     {
-        const NearPair e = work[i];
-        const unsigned char *seg = blob + segs[e.segment].offset;
-        const long long p = e.point;
+        const long long p = listed ? work[i].point : (long long)i;
+        if (listed && i > 0 && work[i - 1].point == (int)p)
+            continue;  // not the first entry of its run
+        const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
         double acc[W];
 #pragma unroll
         for (int k = 0; k < W; ++k)
             acc[k] = 0.0;
-        integrateSegment64<FIELD, 32>(seg, points[3 * p], points[3 * p + 1], points[3 * p + 2], lane, acc);
+        bool any = false;
+        for (unsigned long long e = listed ? i : 0; e < (listed ? n : (unsigned long long)nseg); ++e)
+        {
+            if (listed && work[e].point != (int)p)
+                break;
+            const int s = listed ? work[e].segment : (int)e;
+            if (!listed && !isNearPair(blob, segs, s, px, py, pz))
+                continue;
+            integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
+            any = true;
+        }
+        if (!any)
+            continue;
 #pragma unroll
         for (int off = 16; off > 0; off /= 2)
 #pragma unroll
@@ -292,7 +357,7 @@ __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__re
         {
 #pragma unroll
             for (int k = 0; k < W; ++k)
-                atomicAdd(&out[W * p + k], acc[k]);
+                out[W * p + k] += acc[k];
         }
     }
 }

@@ -65,3 +65,27 @@ def test_pieces_in_fp32_modes(ccoil, mode, points):
             e = e[~gradient_band(rows, pts)]
         assert e.max() < 1e-5, (field, e.max())
         assert np.median(e) < 3e-7, (field, np.median(e))
+
+
+def test_more_near_pairs_than_the_list_holds(ccoil):
+    # the allocation-free entry point's list is far shorter than these points' pairs
+    # (every point lies in the winding box of all 12 coils); the plan's holds them
+    import ctypes
+    import torch
+    coils = [ccoil.Coil(0.1, 0.02, 0.05, 10 + i, 1.0 + i) for i in range(12)]
+    g = np.random.default_rng(5)
+    n = 40003
+    r, phi = g.uniform(0.095, 0.125, n), g.uniform(0.0, 2.0 * np.pi, n)
+    pts = np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, n)], axis=1)
+    x = torch.from_numpy(pts).cuda()
+    L = ccoil.lib()
+    fn = L.ccoil_fields_fp32c_static
+    fn.argtypes = [ctypes.POINTER(ccoil._lib.CoilStruct), ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong,
+                   ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+    structs = (ccoil._lib.CoilStruct * len(coils))(*[c.struct() for c in coils])
+    for field, width in ((0, 3), (1, 3), (3, 9)):
+        want = ccoil.FieldPlan(list(structs), field, ccoil.PrecisionMode.FP32_COMPENSATED)(x).cpu().numpy()
+        out = torch.full((n, width), float("nan"), dtype=torch.float64, device="cuda")
+        assert fn(structs, len(coils), ctypes.c_void_p(x.data_ptr()), n, field, ctypes.c_void_p(out.data_ptr()),
+                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, L.ccoil_last_error_message()
+        assert rel_err(out.cpu().numpy(), want).max() < TOL, field
