@@ -127,151 +127,182 @@ __device__ __forceinline__ bool zAxisCase(const double *pp, const double *sp, do
            fabs(sp[1] / primR) < 1e-12 && fabs(pp[3] / (2 * kPi)) < 1e-12 && fabs(sp[3] / (2 * kPi)) < 1e-12;
 }
 
-// A_phi of the primary at a point and its derivatives in r and z (coil frame):
-//   fast node  a = r' c [asinh(top/rho) - asinh(bot/rho)],
-//              da/dz = r' c (g1 - g2),  da/dr = -r' c (r - r' c)(top g1 - bot g2) / rho^2
-//   slow node  a = r' c / sqrt(D),  da/dz = -r' c zl D^-3/2,  da/dr = -r' c (r - r' c) D^-3/2
-// (the value `a` uses the reference's operation sequence, as segmentA64)
-__device__ __forceinline__ void segmentAGrad64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                               const double2 *pt, const Frame &f, double &A, double &Ar, double &Az)
+// sum over the LANES neighbouring lanes that share a secondary node
+template <int LANES> __device__ __forceinline__ double laneSum(double v)
 {
-    A = segmentA64<1>(h, tt, lt, pt, f, 0);
-    Ar = 0.0;
-    Az = 0.0;
-    const double r = f.r;
-    if (h.fast)
-    {
-        const double top = f.z + h.half_length, bot = f.z - h.half_length;
-        for (int j = 0; j < h.n_t; ++j)
-        {
-            const double2 t = tt[j];
-            double sr = 0.0, sz = 0.0;
-            for (int k = 0; k < h.n_phi; ++k)
-            {
-                const double2 q = pt[k];
-                const double c = q.x;
-                const double rho2 = t.x * t.x + r * r - 2.0 * t.x * r * c;
-                const double g1 = rsqrt(rho2 + top * top), g2 = rsqrt(rho2 + bot * bot);
-                sz += q.y * c * (g1 - g2);
-                sr -= q.y * c * (r - t.x * c) * (top * g1 - bot * g2) / rho2;
-            }
-            Ar += t.y * t.x * sr;
-            Az += t.y * t.x * sz;
-        }
-    }
-    else
-    {
-        for (int i = 0; i < h.n_l; ++i)
-        {
-            const double2 l = lt[i];
-            const double zl = l.x + f.z;
-            for (int j = 0; j < h.n_t; ++j)
-            {
-                const double2 t = tt[j];
-                double sr = 0.0, sz = 0.0;
-                for (int k = 0; k < h.n_phi; ++k)
-                {
-                    const double2 q = pt[k];
-                    const double c = q.x;
-                    const double D = t.x * t.x + r * r - 2.0 * t.x * r * c + zl * zl;
-                    const double g = rsqrt(D), g3 = g * g * g;
-                    sz -= q.y * c * zl * g3;
-                    sr -= q.y * c * (r - t.x * c) * g3;
-                }
-                Ar += l.y * t.y * t.x * sr;
-                Az += l.y * t.y * t.x * sz;
-            }
-        }
-    }
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off /= 2)
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
 }
 
-// Derivatives of the primary's A_phi(r, z) at one point (coil frame) for the
-// parameter gradient, given its value a: with respect to r and z (for the
-// Jacobian) and to the primary's inner radius R, thickness a and length b.
-// With the current density N I / (a b) folded into the node weights, the
-// thickness integral (a / 2) sum w_i f(r'_i) makes the weights independent of
+// Sums of one angular loop of segmentAD64: weighted by w c, the node's value
+// (analytic length integral V, or g) and its derivatives' parts
+struct ADSums
+{
+    double v = 0.0, z = 0.0, r = 0.0, p = 0.0, b = 0.0;
+};
+
+// Fast method: nodes phi and pi - phi together, since a mirror pair takes one
+// logarithm (as phiLoopA64, integrands64f.cuh, whose num / den form of
+// V = asinh(top / rho) - asinh(bot / rho) this is)
+template <bool PARAMS, bool CHECKED, int LANES>
+__device__ __forceinline__ ADSums phiLoopAD64(const double2 *pt, int n, int lane, double p, double r, double top,
+                                              double bot)
+{
+    const double cF = 2.0 * p * r, cC = p * p + r * r, T2 = top * top, B2 = bot * bot;
+    const double aT = fabs(top), aB = fabs(bot);
+    const bool above = bot >= 0.0, below = top < 0.0;
+    ADSums S;
+    auto node = [&](const double2 q, double &num, double &den) {
+        const double c = q.x, wc = q.y * c;
+        const double rho2 = fma(-cF, c, cC);
+        const double x1 = rho2 + T2, x2 = rho2 + B2;
+        const double g1 = rsqrt64t<CHECKED>(x1), g2 = rsqrt64t<CHECKED>(x2);
+        const double a1 = fma(x1, g1, aT), a2 = fma(x2, g2, aB);
+        num = above ? a1 : (below ? a2 : a1 * a2);
+        den = above ? a2 : (below ? a1 : rho2);
+        const double tg = fma(top, g1, -bot * g2);
+        const double wy = wc * (CHECKED ? tg / rho2 : tg * rcp64u(rho2));
+        S.z = fma(wc, g1 - g2, S.z);
+        S.r = fma(wy, fma(-p, c, r), S.r);
+        if (PARAMS)
+        {
+            S.p = fma(wy, fma(-r, c, p), S.p);
+            S.b = fma(wc, g1 + g2, S.b);
+        }
+    };
+#pragma unroll 1
+    for (int m = lane; m < n / 2; m += LANES)
+    {
+        const double2 q = pt[m], qm = pt[n - 1 - m];
+        double n1, e1, n2, e2;
+        node(q, n1, e1);
+        node(qm, n2, e2);
+        S.v = fma(0.5 * (q.y * q.x - qm.y * qm.x), logRatio64t<CHECKED>(n1 * e2, e1 * n2), S.v);
+    }
+    if ((n & 1) && lane == 0)
+    {
+        const double2 q = pt[n / 2];
+        double n1, e1;
+        node(q, n1, e1);
+        S.v = fma(q.y * q.x, logRatio64t<CHECKED>(n1, e1), S.v);
+    }
+    return S;
+}
+
+template <bool PARAMS, bool CHECKED, int LANES>
+__device__ __forceinline__ ADSums phiLoopSlowAD64(const double2 *pt, int n, int lane, double p, double r, double zl2)
+{
+    const double cF = 2.0 * p * r, cD = p * p + r * r + zl2;
+    ADSums S;
+#pragma unroll 2
+    for (int k = lane; k < n; k += LANES)
+    {
+        const double2 q = pt[k];
+        const double c = q.x, wc = q.y * c;
+        const double g = rsqrt64t<CHECKED>(fma(-cF, c, cD));
+        const double wg = wc * g, wg3 = wg * (g * g);
+        S.v += wg;
+        S.z += wg3;
+        S.r = fma(wg3, fma(-p, c, r), S.r);
+        if (PARAMS)
+            S.p = fma(wg3, fma(-r, c, p), S.p);
+    }
+    return S;
+}
+
+// A_phi of the primary at one point (coil frame) and its derivatives: in r and z
+// (for the Jacobian), and with PARAMS by the primary's inner radius R, thickness a
+// and length b.  With the current density N I / (a b) folded into the node weights,
+// the thickness integral (a / 2) sum w_i f(r'_i) makes the weights independent of
 // a, so d/dR = sum w_i df/dr', d/da = sum w_i u_i df/dr' (u_i = dr'_i/da), and
 // for the fast method d/db = -a/b + the derivative of the length limits
 // (top, bot = z +- b/2); for the slow method d/db moves the length nodes.
 //   fast node  f = r' c V,  V = asinh(top/rho) - asinh(bot/rho)
-//              df/dr' = c V - r' c (r' - r c)(top g1 - bot g2) / rho^2,  dV/db = (g1 + g2) / 2
+//              df/dz = r' c (g1 - g2),  df/dr = -r' c (r - r' c) y,
+//              df/dr' = c V - r' c (r' - r c) y,  dV/db = (g1 + g2) / 2,
+//              y = (top g1 - bot g2) / rho^2
 //   slow node  f = r' c g,  g = D^-1/2
-//              df/dr' = c g - r' c (r' - r c) g^3,  df/dzl = -r' c zl g^3
-// out: {dA/dr, dA/dz, dA/dR, dA/da, dA/db}
-__device__ __noinline__ void segmentAParams64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                              const double2 *pt, const double2 *tu, const double2 *lu,
-                                              const Frame &f, double a, double *out)
+//              df/dz = df/dzl = -r' c zl g^3,  df/dr = -r' c (r - r' c) g^3,
+//              df/dr' = c g - r' c (r' - r c) g^3
+// One loop yields all of them: the roots and the reciprocal are shared, 47
+// FP64-pipe operations per fast node where a loop for the value, in the
+// reference's sequence, and one with two asinh and CUDA's rsqrt for the
+// derivatives took about 250.  LANES neighbouring lanes split the angular nodes
+// and every one of them returns their sums.
+// out: {A, dA/dr, dA/dz, dA/dR, dA/da, dA/db} (the first three without PARAMS)
+template <bool PARAMS, int LANES>
+__device__ __noinline__ void segmentAD64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
+                                         const double2 *pt, const double2 *tu, const double2 *lu, double z, double r,
+                                         int lane, double *out)
 {
-    const double r = f.r;
-    double Ar = 0.0, Az = 0.0, dR = 0.0, dA = 0.0, dB = 0.0;
+    double A = 0.0, Ar = 0.0, Az = 0.0, dR = 0.0, dA = 0.0, dB = 0.0;
+    const int n = h.n_phi;
     if (h.fast)
     {
-        const double top = f.z + h.half_length, bot = f.z - h.half_length;
+        const double top = z + h.half_length, bot = z - h.half_length;
         for (int j = 0; j < h.n_t; ++j)
         {
             const double2 t = tt[j];
-            const double p = t.x;
-            double sr = 0.0, sz = 0.0, sp = 0.0, sb = 0.0;
-            for (int k = 0; k < h.n_phi; ++k)
+            const double p = t.x, k = 2.0 * p * r, cC = p * p + r * r;
+            // every root's argument lies in [cC - k, max(top^2, bot^2) + cC + k]
+            const ADSums S = inRange64(cC - k, fmax(top * top, bot * bot) + (cC + k))
+                                 ? phiLoopAD64<PARAMS, false, LANES>(pt, n, lane, p, r, top, bot)
+                                 : phiLoopAD64<PARAMS, true, LANES>(pt, n, lane, p, r, top, bot);
+            A += t.y * p * S.v;
+            Ar -= t.y * p * S.r;
+            Az += t.y * p * S.z;
+            if (PARAMS)
             {
-                const double2 q = pt[k];
-                const double c = q.x;
-                const double rho2 = p * p + r * r - 2.0 * p * r * c;
-                const double g1 = rsqrt(rho2 + top * top), g2 = rsqrt(rho2 + bot * bot);
-                const double irho = rsqrt(rho2);
-                const double V = asinh(top * irho) - asinh(bot * irho);
-                const double tg = top * g1 - bot * g2;
-                sz += q.y * c * (g1 - g2);
-                sr -= q.y * c * (r - p * c) * tg / rho2;
-                sp += q.y * c * (V - p * (p - r * c) * tg / rho2);
-                sb += q.y * c * 0.5 * (g1 + g2);
+                const double sp = t.y * (S.v - p * S.p);
+                dR += sp;
+                dA += tu[j].x * sp;
+                dB += t.y * p * 0.5 * S.b;
             }
-            Ar += t.y * p * sr;
-            Az += t.y * p * sz;
-            dR += t.y * sp;
-            dA += t.y * tu[j].x * sp;
-            dB += t.y * p * sb;
         }
-        dB -= a / (2.0 * h.half_length);
+        if (PARAMS)
+            dB -= A / (2.0 * h.half_length);
     }
     else
     {
         for (int i = 0; i < h.n_l; ++i)
         {
             const double2 l = lt[i];
-            const double zl = l.x + f.z;
+            const double zl = l.x + z, zl2 = zl * zl;
             for (int j = 0; j < h.n_t; ++j)
             {
                 const double2 t = tt[j];
-                const double p = t.x;
-                double sr = 0.0, sz = 0.0, sp = 0.0;
-                for (int k = 0; k < h.n_phi; ++k)
-                {
-                    const double2 q = pt[k];
-                    const double c = q.x;
-                    const double D = p * p + r * r - 2.0 * p * r * c + zl * zl;
-                    const double g = rsqrt(D), g3 = g * g * g;
-                    sz -= q.y * c * zl * g3;
-                    sr -= q.y * c * (r - p * c) * g3;
-                    sp += q.y * (c * g - p * c * (p - r * c) * g3);
-                }
+                const double p = t.x, k = 2.0 * p * r, cD = p * p + r * r + zl2;
+                const ADSums S = inRange64(cD - k, cD + k)
+                                     ? phiLoopSlowAD64<PARAMS, false, LANES>(pt, n, lane, p, r, zl2)
+                                     : phiLoopSlowAD64<PARAMS, true, LANES>(pt, n, lane, p, r, zl2);
                 const double w = l.y * t.y;
-                Ar += w * p * sr;
-                Az += w * p * sz;
-                dR += w * sp;
-                dA += w * tu[j].x * sp;
-                dB += w * lu[i].x * p * sz;
+                A += w * p * S.v;
+                Ar -= w * p * S.r;
+                Az -= w * p * zl * S.z;
+                if (PARAMS)
+                {
+                    const double sp = w * (S.v - p * S.p);
+                    dR += sp;
+                    dA += tu[j].x * sp;
+                    dB -= w * lu[i].x * p * zl * S.z;
+                }
             }
         }
     }
-    out[0] = Ar;
-    out[1] = Az;
-    out[2] = dR;
-    out[3] = dA;
-    out[4] = dB;
+    out[0] = laneSum<LANES>(A);
+    out[1] = laneSum<LANES>(Ar);
+    out[2] = laneSum<LANES>(Az);
+    if (PARAMS)
+    {
+        out[3] = laneSum<LANES>(dR);
+        out[4] = laneSum<LANES>(dA);
+        out[5] = laneSum<LANES>(dB);
+    }
 }
 
-// The same five derivatives with the primary's quadrature in FP32 (mirror
+// The five derivatives of segmentAD64 with the primary's quadrature in FP32 (mirror
 // pairs, two per packed step, differences by subtraction as in the FP32
 // arrangement integrands; the FP64 sum over the secondary's nodes follows).
 // Per node h(c) multiplies c, so a pair adds w c (h(c) - h(-c)):
@@ -458,15 +489,6 @@ struct PairSplit
     int groups = 1, parts = 1;
 };
 
-// sum over the LANES neighbouring lanes that share a secondary node
-template <int LANES> __device__ __forceinline__ double laneSum(double v)
-{
-#pragma unroll
-    for (int off = LANES / 2; off > 0; off /= 2)
-        v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-
 // What a warp needs of its current arrangement and primary, written by lane 0
 // into shared memory and read back by all lanes inside the secondary-node loop
 // (volatile: kept out of registers, which the primary quadrature needs)
@@ -493,12 +515,6 @@ __device__ __forceinline__ Frame frameZR(double z, double r)
     f.cphi = 1.0;
     f.sphi = 0.0;
     return f;
-}
-
-__device__ __noinline__ double pairA64(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                       const double2 *pt, double z, double r)
-{
-    return segmentA64<1>(h, tt, lt, pt, frameZR(z, r), 0);
 }
 
 // The FP32 kernels' FP64 nodes (near-field and refined): FP64 accuracy without
@@ -560,7 +576,7 @@ __device__ __noinline__ double2 pairB32(const SegmentHeader &h, const double2 *t
 // Few arrangements are cut into more work units than one per arrangement: groups
 // of primaries and, within one primary, ranges of its secondary nodes
 // (PairSplit).  Each unit's sums go to `partial` and pairReduceKernel adds an
-// arrangement's units in a fixed order.  LANES > 1 (FP64 M and F/T): that many
+// arrangement's units in a fixed order.  LANES > 1 (FP64 M, F/T and position gradient): that many
 // lanes share a secondary node and split the primary's angular nodes.
 template <int QTY, bool FP32, bool REFINE = false, int LANES = 1>
 __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
@@ -766,18 +782,15 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                     const double2 *lu = reinterpret_cast<const double2 *>(base) + ph.off_lu;
                     const double ul = (reinterpret_cast<const double2 *>(base) + ph.off_slu)[l].x;
                     const double ut = (reinterpret_cast<const double2 *>(base) + ph.off_stu)[t].x;
-                    double av, d[5];
+                    double ad[6], *d = ad + 1;
                     if (FP32 && far)
                     {
-                        av = pairA32(h, tt, lt, pn, f.z, f.r);
-                        segmentAParams32(h, tt, lt, pn, tu, lu, f, av, d);
+                        ad[0] = pairA32(h, tt, lt, pn, f.z, f.r);
+                        segmentAParams32(h, tt, lt, pn, tu, lu, f, ad[0], d);
                     }
                     else
-                    {
-                        av = pairA64(h, tt, lt, pt, f.z, f.r);
-                        segmentAParams64(h, tt, lt, pt, tu, lu, f, av, d);
-                    }
-                    const double ar = d[0], az = d[1];
+                        segmentAD64<true, LANES>(h, tt, lt, pt, tu, lu, f.z, f.r, sub, ad);
+                    const double av = ad[0], ar = d[0], az = d[1];
                     const double c = f.cphi, s_ = f.sphi;
                     const double ao = f.r > 0.0 ? av / f.r : ar;
                     const double J[9] = {s_ * c * (ao - ar), -s_ * s_ * ar - c * c * ao, -s_ * az,
@@ -849,8 +862,9 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                 {
                     // dM/d(secondary position) = factor sum_n w_n J_A(q_n)^T t_n,
                     // J_A = T J_loc T^T; J_loc of A_loc = a(r, z) (-sin, cos, 0)
-                    double av, ar, az;
-                    segmentAGrad64(h, tt, lt, pt, f, av, ar, az);
+                    double ad[3];
+                    segmentAD64<false, LANES>(h, tt, lt, pt, nullptr, nullptr, f.z, f.r, sub, ad);
+                    const double av = ad[0], ar = ad[1], az = ad[2];
                     const double c = f.cphi, s_ = f.sphi;
                     const double ao = f.r > 0.0 ? av / f.r : ar;
                     const double J[9] = {s_ * c * (ao - ar), -s_ * s_ * ar - c * c * ao, -s_ * az,
@@ -1423,8 +1437,11 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     int lanes = 1;
     if (!refine)
     {
-        // fewer warp iterations in all than resident warps: 8 lanes share a secondary node
-        if (!fp32 && quantity <= CCOIL_PAIR_FORCE_TORQUE && count * primary_count * ((secNodes + 31) / 32) < resident)
+        // fewer warp iterations in all than resident warps: 8 lanes share a secondary
+        // node (not for the parameter gradient, some of whose columns vanish by
+        // symmetry: a node evaluated by one lane leaves the same rounding in them
+        // however the arrangement is cut)
+        if (!fp32 && quantity != CCOIL_PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT && count * primary_count * ((secNodes + 31) / 32) < resident)
             lanes = 8;
         split = pairSplit(count, primary_count, secNodes, 32 / lanes, resident);
     }
@@ -1470,6 +1487,8 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         CCOIL_PAIR_LAUNCH(0, false, false, 8);
     else if (quantity == CCOIL_PAIR_FORCE_TORQUE && !fp32 && lanes == 8)
         CCOIL_PAIR_LAUNCH(1, false, false, 8);
+    else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE_GRADIENT && lanes == 8)
+        CCOIL_PAIR_LAUNCH(2, false, false, 8);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32)
         CCOIL_PAIR_LAUNCH(0, false);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && refine)
