@@ -88,6 +88,99 @@ __device__ __forceinline__ void matTvec(const double *M, const double *v, double
     o[2] = M[2] * v[0] + M[5] * v[1] + M[8] * v[2];
 }
 
+#include "fp64ops.cuh"
+
+// The sums of one angular loop.  Fast method, each weighted by w (and the ones
+// marked c by w c): with D3 = g1^3 - g2^3, T3 = top g1^3 - bot g2^3,
+// Y = (top g1 - bot g2) / rho^2 and m = r' - r c (so N = r' m),
+//   a0 c (g2 - g1)     a1 m Y          a2 c D3 m       a3 Y
+//   a4 m (m / rho^2) (T3 + 2 Y)        a5 c (top g1^3 + bot g2^3)
+//   a6 m (g1^3 + g2^3) a7 c D3 (r - r' c)              a8 c T3    a9 m D3
+// from which dZ/dr' = r' a3 + a1 - r' a4 (the node's form above, with
+// 2 r' - r c = r' + m), and the other terms by factors of r' alone.
+// Slow method (G3 = G^3, G5 = G^5):
+//   a0 c G3  a1 m G3  a2 c m G5  a3 G3  a4 m m G5  a5 c G5  a6 m G5  a7 c G5 (r - r' c)
+struct AdjSums
+{
+    double a[10];
+};
+
+// One fast node costs 49 FP64-pipe operations this way; with the terms formed one
+// by one, CUDA's reciprocal roots and IEEE divisions it took 133.  The FP64 pipe
+// bounds the kernel: 64 RECTANGULAR coils at 4,096 points 3.54 -> 1.61 ms, 128
+// mixed coils at 200,000 points 129 -> 61.6 ms (81 % of that pipe's measured rate;
+// two nodes in flight per thread, and register caps of 168, 128 and 96 measured
+// slower than the compiler's own choice).  Arguments outside [kLo64, kHi64] take
+// the IEEE operations (CHECKED).
+template <bool CHECKED>
+__device__ __forceinline__ void adjFastLoop(const double2 *pt, int n, int lane, double rp, double r, double top,
+                                            double bot, AdjSums &S)
+{
+    const double cF = 2.0 * rp * r, cC = rp * rp + r * r, T2 = top * top, B2 = bot * bot;
+#pragma unroll 2
+    for (int k = lane; k < n; k += kAdjLanes)
+    {
+        const double2 q = pt[k];
+        const double c = q.x, w = q.y, wc = w * c;
+        const double rho2 = fma(-cF, c, cC);
+        const double g1 = rsqrt64t<CHECKED>(rho2 + T2), g2 = rsqrt64t<CHECKED>(rho2 + B2);
+        const double i = CHECKED ? 1.0 / rho2 : rcp64u(rho2);
+        const double g13 = g1 * (g1 * g1), g23 = g2 * (g2 * g2);
+        const double D3 = g13 - g23, t1 = top * g13, t2 = bot * g23, T3 = t1 - t2;
+        const double Y = fma(top, g1, -bot * g2) * i;
+        const double m = fma(-r, c, rp), wm = w * m, wcD = wc * D3;
+        S.a[0] = fma(wc, g2 - g1, S.a[0]);
+        S.a[1] = fma(wm, Y, S.a[1]);
+        S.a[2] = fma(wcD, m, S.a[2]);
+        S.a[3] = fma(w, Y, S.a[3]);
+        S.a[4] = fma(wm * (m * i), fma(2.0, Y, T3), S.a[4]);
+        S.a[5] = fma(wc, t1 + t2, S.a[5]);
+        S.a[6] = fma(wm, g13 + g23, S.a[6]);
+        S.a[7] = fma(wcD, fma(-rp, c, r), S.a[7]);
+        S.a[8] = fma(wc, T3, S.a[8]);
+        S.a[9] = fma(wm, D3, S.a[9]);
+    }
+}
+
+template <bool CHECKED>
+__device__ __forceinline__ void adjSlowLoop(const double2 *pt, int n, int lane, double rp, double r, double zl2,
+                                            AdjSums &S)
+{
+    const double cF = 2.0 * rp * r, cD = rp * rp + r * r + zl2;
+#pragma unroll 2
+    for (int k = lane; k < n; k += kAdjLanes)
+    {
+        const double2 q = pt[k];
+        const double c = q.x, w = q.y, wc = w * c;
+        const double G = rsqrt64t<CHECKED>(fma(-cF, c, cD));
+        const double G2 = G * G, G3 = G2 * G, G5 = G3 * G2;
+        const double m = fma(-r, c, rp), wm = w * m, wcG5 = wc * G5, wmG5 = wm * G5;
+        S.a[0] = fma(wc, G3, S.a[0]);
+        S.a[1] = fma(wm, G3, S.a[1]);
+        S.a[2] = fma(wcG5, m, S.a[2]);
+        S.a[3] = fma(w, G3, S.a[3]);
+        S.a[4] = fma(wmG5, m, S.a[4]);
+        S.a[5] += wcG5;
+        S.a[6] += wmG5;
+        S.a[7] = fma(wcG5, fma(-rp, c, r), S.a[7]);
+    }
+}
+
+__device__ __noinline__ AdjSums adjFastIeee(const double2 *pt, int n, int lane, double rp, double r, double top,
+                                            double bot)
+{
+    AdjSums S = {};
+    adjFastLoop<true>(pt, n, lane, rp, r, top, bot, S);
+    return S;
+}
+
+__device__ __noinline__ AdjSums adjSlowIeee(const double2 *pt, int n, int lane, double rp, double r, double zl2)
+{
+    AdjSums S = {};
+    adjSlowLoop<true>(pt, n, lane, rp, r, zl2, S);
+    return S;
+}
+
 __global__ void __launch_bounds__(kAdjThreads) adjointKernel(const unsigned char *__restrict__ blob,
                                                              const long long *__restrict__ offsets, int ncoils,
                                                              const double *__restrict__ points,
@@ -126,48 +219,28 @@ __global__ void __launch_bounds__(kAdjThreads) adjointKernel(const unsigned char
             for (int j = 0; j < C.nt; ++j)
             {
                 const AdjT t = tt[j];
-                const double rp = t.rp;
-                double a[10];
-                for (int i = 0; i < 10; ++i)
-                    a[i] = 0.0;
-                for (int k = lane; k < C.nphi; k += kAdjLanes)
-                {
-                    const double2 q = pt[k];
-                    const double cc = q.x, w = q.y;
-                    const double rho2 = rp * rp + r * r - 2.0 * rp * r * cc;
-                    const double g1 = rsqrt(rho2 + top * top), g2 = rsqrt(rho2 + bot * bot);
-                    const double g13 = g1 * g1 * g1, g23 = g2 * g2 * g2;
-                    const double N = rp * rp - rp * r * cc, E = top * g1 - bot * g2;
-                    const double hH = rp * cc * (g2 - g1), hZ = N / rho2 * E;
-                    const double rmc = rp - r * cc;
-                    const double dHdr = cc * (g2 - g1) + rp * cc * rmc * (g13 - g23);
-                    const double dE = -rmc * (top * g13 - bot * g23);
-                    const double dZdr = ((2.0 * rp - r * cc) * E + N * dE) / rho2 - 2.0 * N * E * rmc / (rho2 * rho2);
-                    const double dHdb = 0.5 * (rp * cc * top * g13 + rp * cc * bot * g23);
-                    const double dZdb = 0.5 * (N * g13 + N * g23);
-                    a[0] += w * hH;
-                    a[1] += w * hZ;
-                    a[2] += w * dHdr;
-                    a[3] += w * dZdr;
-                    a[4] += w * dHdb;
-                    a[5] += w * dZdb;
-                    a[6] += w * hH;                                     // RPhi * r
-                    a[7] += w * rp * cc * (r - rp * cc) * (g13 - g23);  // RR
-                    a[8] += w * rp * cc * (top * g13 - bot * g23);      // RZ
-                    a[9] += w * N * (g13 - g23);                        // ZZ
-                }
-                s[0] += t.w * a[0];
-                s[1] += t.w * a[1];
-                s[2] += t.w * a[2];
-                s[3] += t.w * a[3];
-                s[4] += t.w * t.u * a[2];
-                s[5] += t.w * t.u * a[3];
-                s[6] += t.w * a[4];
-                s[7] += t.w * a[5];
-                s[8] += t.w * a[6];
-                s[9] += t.w * a[7];
-                s[10] += t.w * a[8];
-                s[11] += t.w * a[9];
+                const double rp = t.rp, k = 2.0 * rp * r, cC = rp * rp + r * r;
+                AdjSums S = {};
+                if (inRange64(cC - k, fmax(top * top, bot * bot) + (cC + k)))
+                    adjFastLoop<false>(pt, C.nphi, lane, rp, r, top, bot, S);
+                else
+                    S = adjFastIeee(pt, C.nphi, lane, rp, r, top, bot);
+                const double *a = S.a;
+                const double H = t.w * rp * a[0];
+                const double dH = t.w * fma(rp, a[2], a[0]), dZ = t.w * (fma(rp, a[3] - a[4], a[1]));
+                const double wp = t.w * rp;
+                s[0] += H;
+                s[1] += wp * a[1];
+                s[2] += dH;
+                s[3] += dZ;
+                s[4] += t.u * dH;
+                s[5] += t.u * dZ;
+                s[6] += 0.5 * wp * a[5];
+                s[7] += 0.5 * wp * a[6];
+                s[8] += H;  // RPhi * r
+                s[9] += wp * a[7];
+                s[10] += wp * a[8];
+                s[11] += wp * a[9];
             }
         else
         {
@@ -179,40 +252,31 @@ __global__ void __launch_bounds__(kAdjThreads) adjointKernel(const unsigned char
                 for (int j = 0; j < C.nt; ++j)
                 {
                     const AdjT t = tt[j];
-                    const double rp = t.rp;
-                    double a[8];
-                    for (int i = 0; i < 8; ++i)
-                        a[i] = 0.0;
-                    for (int k = lane; k < C.nphi; k += kAdjLanes)
-                    {
-                        const double2 q = pt[k];
-                        const double cc = q.x, w = q.y;
-                        const double G = rsqrt(rp * rp + r * r + zl * zl - 2.0 * rp * r * cc);
-                        const double G3 = G * G * G, G5 = G3 * G * G;
-                        const double N = rp * rp - rp * r * cc, rmc = rp - r * cc;
-                        const double hH = rp * cc * zl * G3;
-                        a[0] += w * hH;
-                        a[1] += w * N * G3;
-                        a[2] += w * (cc * zl * G3 - 3.0 * rp * cc * zl * rmc * G5);
-                        a[3] += w * ((2.0 * rp - r * cc) * G3 - 3.0 * N * rmc * G5);
-                        a[4] += w * (rp * cc * G3 - 3.0 * rp * cc * zl * zl * G5);  // dH/dzl = RZ
-                        a[5] += w * (-3.0 * N * zl * G5);                         // dZ/dzl = ZZ
-                        a[6] += w * hH;                                           // RPhi * r
-                        a[7] += w * (-3.0 * rp * cc * zl * (r - rp * cc) * G5);   // RR
-                    }
-                    const double lw = L.w * t.w;
-                    s[0] += lw * a[0];
-                    s[1] += lw * a[1];
-                    s[2] += lw * a[2];
-                    s[3] += lw * a[3];
-                    s[4] += lw * t.u * a[2];
-                    s[5] += lw * t.u * a[3];
-                    s[6] += lw * L.u * a[4];
-                    s[7] += lw * L.u * a[5];
-                    s[8] += lw * a[6];
-                    s[9] += lw * a[7];
-                    s[10] += lw * a[4];
-                    s[11] += lw * a[5];
+                    const double rp = t.rp, k = 2.0 * rp * r, cD = rp * rp + r * r + zl * zl;
+                    AdjSums S = {};
+                    if (inRange64(cD - k, cD + k))
+                        adjSlowLoop<false>(pt, C.nphi, lane, rp, r, zl * zl, S);
+                    else
+                        S = adjSlowIeee(pt, C.nphi, lane, rp, r, zl * zl);
+                    const double *a = S.a;
+                    const double lw = L.w * t.w, wp = lw * rp;
+                    const double H = wp * zl * a[0];
+                    const double dH = lw * zl * fma(-3.0 * rp, a[2], a[0]);
+                    const double dZ = lw * (fma(rp, a[3], a[1]) - 3.0 * rp * a[4]);
+                    const double RZ = wp * fma(-3.0 * zl * zl, a[5], a[0]);  // dH/dzl
+                    const double ZZ = -3.0 * wp * zl * a[6];                 // dZ/dzl
+                    s[0] += H;
+                    s[1] += wp * a[1];
+                    s[2] += dH;
+                    s[3] += dZ;
+                    s[4] += t.u * dH;
+                    s[5] += t.u * dZ;
+                    s[6] += L.u * RZ;
+                    s[7] += L.u * ZZ;
+                    s[8] += H;  // RPhi * r
+                    s[9] -= 3.0 * wp * zl * a[7];
+                    s[10] += RZ;
+                    s[11] += ZZ;
                 }
             }
         }
@@ -296,16 +360,29 @@ __global__ void __launch_bounds__(kAdjThreads) adjointKernel(const unsigned char
     }
 }
 
-// fixed-order sum of the CTA partials
-__global__ void adjointReduce(const double *__restrict__ partial, int blocks, int ncoils, double *__restrict__ out)
+// Sum of the CTA partials in a fixed order: a block takes 32 values, its 32 rows of
+// threads every 32nd CTA's each
+__global__ void __launch_bounds__(1024) adjointReduce(const double *__restrict__ partial, int blocks, int ncoils,
+                                                      double *__restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ncoils * 9)
-        return;
+    __shared__ double rows[32][32];
+    const int x = threadIdx.x % 32, y = threadIdx.x / 32, n = ncoils * 9;
+    const int i = blockIdx.x * 32 + x;
     double s = 0.0;
-    for (int b = 0; b < blocks; ++b)
-        s += partial[(long long)b * ncoils * 9 + i];
-    out[i] = s;
+    if (i < n)
+    {
+#pragma unroll 4
+        for (int b = y; b < blocks; b += 32)
+            s += partial[(long long)b * n + i];
+    }
+    rows[y][x] = s;
+    __syncthreads();
+    if (y == 0 && i < n)
+    {
+        for (int r = 1; r < 32; ++r)
+            s += rows[r][x];
+        out[i] = s;
+    }
 }
 
 void putBytes(std::vector<unsigned char> &blob, const void *p, size_t n)
@@ -452,7 +529,7 @@ extern "C" int ccoil_b_field_adjoint(const double *params, const ccoil_precision
     if (e == cudaSuccess)
         e = cudaGetLastError();
     if (e == cudaSuccess)
-        adjointReduce<<<(coil_count * 9 + 255) / 256, 256, 0, st>>>(static_cast<const double *>(dPartial.p),
+        adjointReduce<<<(coil_count * 9 + 31) / 32, 1024, 0, st>>>(static_cast<const double *>(dPartial.p),
                                                                     (int)blocks, coil_count, grad_params);
     if (e == cudaSuccess)
         e = cudaGetLastError();

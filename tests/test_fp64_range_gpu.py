@@ -50,3 +50,52 @@ def test_points_on_the_winding_radius(ccoil, oracle, field, lanes):
     plan.close()
     e = rel_err(got, oracle.coil_fields(row, pts, field, pf=5.0))
     assert e.max() < TOL, e.max()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-10, 3e-18, 1e-21, 1e10, 3e17])
+def test_adjoint_is_scale_invariant(ccoil, scale):
+    """B falls as 1 / length: with every length scaled by s, dB/d(length) scales by
+    s^-2 and dB/d(N I), dB/d(angle) by 1 / s.  The parameter gradient at the scaled
+    geometry, inside, across and outside the range of the forms, against the
+    unscaled one (bar 1e-11 of each parameter's scale: the forms differ by a few
+    roundings per node, the points' coordinates by one)."""
+    import torch
+    from ccoil_b200 import autograd, workloads
+    rows, pts = workloads.adjoint_config(coils=6, points=333, seed=41, types=(0, 1, 2, 3))
+    q = np.stack([rows[:, 0], rows[:, 1], rows[:, 2], rows[:, 3] * rows[:, 4], *rows[:, 6:11].T], axis=1)
+    v = np.random.default_rng(42).normal(size=pts.shape)
+
+    def grad(s):
+        p = q.copy()
+        p[:, [0, 1, 2, 4, 5, 6]] *= s
+        P = torch.tensor(p, requires_grad=True)
+        B = autograd.b_field(P, torch.from_numpy(pts * s).cuda(), autograd.precisions_for(q))
+        (B * torch.from_numpy(v).cuda()).sum().backward()
+        g = P.grad.numpy() * s
+        g[:, [0, 1, 2, 4, 5, 6]] *= s
+        g[:, 1][q[:, 1] == 0.0] = 0.0  # a zero dimension is 1e-25 R at any scale
+        g[:, 2][q[:, 2] == 0.0] = 0.0
+        return g
+
+    want = grad(1.0)
+    assert np.max(np.abs(grad(scale) - want) / np.abs(want).max(axis=0)) < 1e-11
+
+
+@pytest.mark.parametrize("points", [1, 31, 1025, 70001])
+def test_adjoint_sums_over_points(ccoil, points):
+    """The gradient over all points is the sum over two halves (bar 1e-12 of each
+    parameter's scale: FP64 sums in another order)."""
+    import torch
+    from ccoil_b200 import autograd, workloads
+    rows, pts = workloads.adjoint_config(coils=4, points=points, seed=43, types=(0, 2, 1, 3))
+    q = np.stack([rows[:, 0], rows[:, 1], rows[:, 2], rows[:, 3] * rows[:, 4], *rows[:, 6:11].T], axis=1)
+    precs = autograd.precisions_for(q, 3.0)
+
+    def grad(x):
+        P = torch.tensor(q, requires_grad=True)
+        (autograd.b_field(P, torch.from_numpy(x).cuda(), precs) ** 2).sum().backward()
+        return P.grad.numpy()
+
+    whole, half = grad(pts), points // 2
+    parts = grad(pts[:half]) + grad(pts[half:])
+    assert np.max(np.abs(parts - whole) / np.abs(whole).max(axis=0)) < 1e-12
