@@ -8,8 +8,10 @@
 // list is exhausted, so long items start first and short ones fill the tail.
 // An item reads its system's segment tables straight from global memory
 // (through L1, as the single-system kernels do), so warps synchronise only to
-// take the next item.  In FP32_COMPENSATED mode near-field pairs go to the
-// work list with the field in the top bits of the segment index.
+// take the next item.  In FP32_COMPENSATED mode the items leave near-field pairs
+// out; a second kernel lists them, a point's next to each other with the field in
+// the top bits of the segment index, and a third evaluates them (as the
+// single-system kernels, fields32.cuh).
 
 struct BatchItem
 {
@@ -27,10 +29,11 @@ constexpr int kFieldShift = 28;  // NearPair.segment = segment | field << 28
 template <int PREC, int FIELD, int LANES>
 __device__ __forceinline__ void batchItem(const BatchItem &I, const unsigned char *__restrict__ blob,
                                           const SegmentDesc *__restrict__ segs, const double *__restrict__ points,
-                                          double *__restrict__ out, NearPair *__restrict__ work,
-                                          unsigned long long workCapacity, unsigned long long *__restrict__ workCount)
+                                          double *__restrict__ out, double (*sums)[128])
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
+    // the FP32 gradient's sums in shared memory, as fieldsKernel32's
+    constexpr bool kShared = FIELD == CCOIL_FIELD_G && PREC != CCOIL_PRECISION_FP64;
     const int lane = threadIdx.x % LANES;
     const int local = threadIdx.x / LANES;
     const bool active = local < I.point_count;
@@ -47,7 +50,11 @@ __device__ __forceinline__ void batchItem(const BatchItem &I, const unsigned cha
     double acc[W];
 #pragma unroll
     for (int i = 0; i < W; ++i)
+    {
         acc[i] = 0.0;
+        if (kShared)
+            sums[kShared ? i : 0][threadIdx.x] = 0.0;
+    }
 
     for (int s = 0; s < nseg && active; ++s)
     {
@@ -58,29 +65,27 @@ __device__ __forceinline__ void batchItem(const BatchItem &I, const unsigned cha
         {
             const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
             const Frame f = toCoilFrame(h, px, py, pz);
-            if (!nearWinding(h, f))
-                integrateSegment32<FIELD, LANES>(seg, f, lane, acc);
-            else
+            if (nearWinding(h, f))
+                continue;
+            if (kShared)
             {
-                bool queued = false;
-                if (lane == 0)
-                {
-                    unsigned long long slot = atomicAdd(workCount, 1ull);
-                    if (slot < workCapacity)
-                    {
-                        work[slot].point = (int)p;
-                        work[slot].segment = (I.seg_begin + s) | (FIELD << kFieldShift);
-                        queued = true;
-                    }
-                }
-                const unsigned groupMask = LANES == 32 ? 0xffffffffu
-                                                       : (((1u << LANES) - 1u) << ((threadIdx.x % 32) / LANES * LANES));
-                queued = __shfl_sync(groupMask, queued, (threadIdx.x % 32) / LANES * LANES);
-                if (!queued)
-                    integrateSegment64Fallback<FIELD, LANES>(seg, px, py, pz, lane, acc);
+                double c[W];
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    c[i] = 0.0;
+                integrateSegment32<FIELD, LANES>(seg, f, lane, c);
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    sums[kShared ? i : 0][threadIdx.x] += c[i];
             }
+            else
+                integrateSegment32<FIELD, LANES>(seg, f, lane, acc);
         }
     }
+    if (kShared)
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            acc[i] = sums[kShared ? i : 0][threadIdx.x];
 #pragma unroll
     for (int off = LANES / 2; off > 0; off /= 2)
 #pragma unroll
@@ -96,14 +101,13 @@ __device__ __forceinline__ void batchItem(const BatchItem &I, const unsigned cha
 
 template <int PREC, int FIELD>
 __device__ __forceinline__ void batchItemLanes(const BatchItem &I, const unsigned char *blob, const SegmentDesc *segs,
-                                               const double *points, double *out, NearPair *work,
-                                               unsigned long long cap, unsigned long long *count)
+                                               const double *points, double *out, double (*sums)[128])
 {
     switch (I.lanes)
     {
-        case 1: batchItem<PREC, FIELD, 1>(I, blob, segs, points, out, work, cap, count); break;
-        case 4: batchItem<PREC, FIELD, 4>(I, blob, segs, points, out, work, cap, count); break;
-        default: batchItem<PREC, FIELD, 32>(I, blob, segs, points, out, work, cap, count); break;
+        case 1: batchItem<PREC, FIELD, 1>(I, blob, segs, points, out, sums); break;
+        case 4: batchItem<PREC, FIELD, 4>(I, blob, segs, points, out, sums); break;
+        default: batchItem<PREC, FIELD, 32>(I, blob, segs, points, out, sums); break;
     }
 }
 
@@ -130,11 +134,10 @@ __global__ void __launch_bounds__(128, batchMinBlocks(PREC)) batchKernel(const u
                                                       const BatchItem *__restrict__ items, int nitems,
                                                       unsigned *__restrict__ next, const double *__restrict__ points,
                                                       double *__restrict__ outA, double *__restrict__ outB,
-                                                      double *__restrict__ outG, NearPair *__restrict__ work,
-                                                      unsigned long long workCapacity,
-                                                      unsigned long long *__restrict__ workCount)
+                                                      double *__restrict__ outG)
 {
     __shared__ int itemIndex;
+    __shared__ double sums[PREC == CCOIL_PRECISION_FP64 ? 1 : 9][128];
     for (;;)
     {
         if (threadIdx.x == 0)
@@ -146,64 +149,139 @@ __global__ void __launch_bounds__(128, batchMinBlocks(PREC)) batchKernel(const u
             break;
         const BatchItem I = items[it];
         if (I.field == CCOIL_FIELD_B)
-            batchItemLanes<PREC, CCOIL_FIELD_B>(I, blob, segs, points, outB, work, workCapacity, workCount);
+            batchItemLanes<PREC, CCOIL_FIELD_B>(I, blob, segs, points, outB, sums);
         else if (I.field == CCOIL_FIELD_G)
-            batchItemLanes<PREC, CCOIL_FIELD_G>(I, blob, segs, points, outG, work, workCapacity, workCount);
+            batchItemLanes<PREC, CCOIL_FIELD_G>(I, blob, segs, points, outG, sums);
         else
-            batchItemLanes<PREC, CCOIL_FIELD_A>(I, blob, segs, points, outA, work, workCapacity, workCount);
+            batchItemLanes<PREC, CCOIL_FIELD_A>(I, blob, segs, points, outA, sums);
     }
 }
 
-// near-field pass of the batched kernel: the field is in the segment's top bits
+// Lists the near-field pairs: a block per item of the lowest field, a thread per
+// point; a point's entries are consecutive, field by field.
+__global__ void __launch_bounds__(128) batchNearListKernel(const unsigned char *__restrict__ blob,
+                                                           const SegmentDesc *__restrict__ segs,
+                                                           const BatchItem *__restrict__ items, int nitems,
+                                                           int fieldsMask, const double *__restrict__ points,
+                                                           NearPair *__restrict__ work,
+                                                           unsigned long long workCapacity,
+                                                           unsigned long long *__restrict__ workCount)
+{
+    const int lowest = __ffs(fieldsMask) - 1, fields = __popc(fieldsMask);
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x)
+    {
+        const BatchItem I = items[it];
+        if (I.field != lowest || threadIdx.x >= I.point_count)
+            continue;
+        const long long p = (long long)I.point_begin + threadIdx.x;
+        const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
+        int count = 0;
+        for (int s = I.seg_begin; s < I.seg_end; ++s)
+            count += isNearPair(blob, segs, s, px, py, pz) ? 1 : 0;
+        if (count == 0)
+            continue;
+        unsigned long long slot = atomicAdd(workCount, (unsigned long long)count * fields);
+        for (int f = lowest; f <= CCOIL_FIELD_G; ++f)
+        {
+            if (!(fieldsMask & (1 << f)))
+                continue;
+            for (int s = I.seg_begin; s < I.seg_end && slot < workCapacity; ++s)
+                if (isNearPair(blob, segs, s, px, py, pz))
+                {
+                    work[slot].point = (int)p;
+                    work[slot].segment = s | (f << kFieldShift);
+                    ++slot;
+                }
+        }
+    }
+}
+
+// One warp: the near-field pairs of one point and field, in segment order, FP64,
+// the lanes splitting the angular nodes.  listed: entries [i, ...) of the list up to
+// the point's or field's last; otherwise all segments of [segBegin, segEnd).
+template <int FIELD>
+__device__ __forceinline__ void batchNearPoint(const unsigned char *blob, const SegmentDesc *segs,
+                                               const double *points, double *out, long long p, bool listed,
+                                               const NearPair *work, unsigned long long i, unsigned long long n,
+                                               int segBegin, int segEnd, int lane)
+{
+    constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
+    const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
+    double acc[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+        acc[k] = 0.0;
+    const unsigned long long end = listed ? n : (unsigned long long)segEnd;
+    for (unsigned long long e = listed ? i : (unsigned long long)segBegin; e < end; ++e)
+    {
+        int s = (int)e;
+        if (listed)
+        {
+            if (work[e].point != (int)p || work[e].segment >> kFieldShift != FIELD)
+                break;
+            s = work[e].segment & ((1 << kFieldShift) - 1);
+        }
+        else if (!isNearPair(blob, segs, s, px, py, pz))
+            continue;
+        integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off /= 2)
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            out[W * p + k] += acc[k];
+}
+
+// Near-field pass of the batched kernel: a warp per run of entries, or, with more
+// pairs than the list holds, per point of each item.
 __global__ void __launch_bounds__(256) batchNearKernel(const unsigned char *__restrict__ blob,
                                                        const SegmentDesc *__restrict__ segs,
+                                                       const BatchItem *__restrict__ items, int nitems,
                                                        const double *__restrict__ points, double *__restrict__ outA,
                                                        double *__restrict__ outB, double *__restrict__ outG,
                                                        const NearPair *__restrict__ work,
                                                        unsigned long long workCapacity,
                                                        const unsigned long long *__restrict__ workCount)
 {
-    const unsigned long long n = min(*workCount, workCapacity);
+    const unsigned long long n = *workCount;
+    const bool listed = n <= workCapacity;
     const int lane = threadIdx.x % 32;
     const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const unsigned long long warps = (unsigned long long)gridDim.x * blockDim.x / 32;
-    for (unsigned long long i = warp; i < n; i += warps)
+    // list entry, or point threadIdx of 128 of an item
+    const unsigned long long end = listed ? n : (unsigned long long)nitems * 128;
+    for (unsigned long long i = warp; i < end; i += warps)
     {
-        const NearPair e = work[i];
-        const int field = e.segment >> kFieldShift;
-        const int segIdx = e.segment & ((1 << kFieldShift) - 1);
-        const unsigned char *seg = blob + segs[segIdx].offset;
-        const long long p = e.point;
-        double acc[9];
-        for (int k = 0; k < 9; ++k)
-            acc[k] = 0.0;
-        const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
-        int W;
-        double *out;
-        if (field == CCOIL_FIELD_G)
+        long long p;
+        int field, segBegin = 0, segEnd = 0;
+        if (listed)
         {
-            integrateSegment64<CCOIL_FIELD_G, 32>(seg, px, py, pz, lane, acc);
-            W = 9;
-            out = outG;
-        }
-        else if (field == CCOIL_FIELD_B)
-        {
-            integrateSegment64<CCOIL_FIELD_B, 32>(seg, px, py, pz, lane, acc);
-            W = 3;
-            out = outB;
+            const NearPair e = work[i];
+            field = e.segment >> kFieldShift;
+            p = e.point;
+            if (i > 0 && work[i - 1].point == e.point && work[i - 1].segment >> kFieldShift == field)
+                continue;  // not the first entry of its run
         }
         else
         {
-            integrateSegment64<CCOIL_FIELD_A, 32>(seg, px, py, pz, lane, acc);
-            W = 3;
-            out = outA;
+            const BatchItem I = items[i / 128];
+            if ((int)(i % 128) >= I.point_count)
+                continue;
+            field = I.field;
+            p = (long long)I.point_begin + (int)(i % 128);
+            segBegin = I.seg_begin;
+            segEnd = I.seg_end;
         }
-        for (int off = 16; off > 0; off /= 2)
-            for (int k = 0; k < 9; ++k)
-                acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        if (lane == 0)
-            for (int k = 0; k < W; ++k)
-                atomicAdd(&out[W * p + k], acc[k]);
+        if (field == CCOIL_FIELD_G)
+            batchNearPoint<CCOIL_FIELD_G>(blob, segs, points, outG, p, listed, work, i, n, segBegin, segEnd, lane);
+        else if (field == CCOIL_FIELD_B)
+            batchNearPoint<CCOIL_FIELD_B>(blob, segs, points, outB, p, listed, work, i, n, segBegin, segEnd, lane);
+        else
+            batchNearPoint<CCOIL_FIELD_A>(blob, segs, points, outA, p, listed, work, i, n, segBegin, segEnd, lane);
     }
 }
 
@@ -221,17 +299,17 @@ int launchBatchImpl(const BatchLaunch &B, cudaStream_t st)
     const BatchItem *items = static_cast<const BatchItem *>(B.d_items);
     if (B.precision == CCOIL_PRECISION_FP64)
         batchKernel<CCOIL_PRECISION_FP64><<<B.grid, 128, 0, st>>>(B.d_blob, B.d_segs, items, B.nitems, B.d_next,
-                                                                     B.d_points, B.d_outA, B.d_outB, B.d_outG, work,
-                                                                     B.work_capacity, B.d_work_count);
+                                                                     B.d_points, B.d_outA, B.d_outB, B.d_outG);
     else
         batchKernel<CCOIL_PRECISION_FP32_COMPENSATED><<<B.grid, 128, 0, st>>>(
-            B.d_blob, B.d_segs, items, B.nitems, B.d_next, B.d_points, B.d_outA, B.d_outB, B.d_outG, work,
-            B.work_capacity, B.d_work_count);
+            B.d_blob, B.d_segs, items, B.nitems, B.d_next, B.d_points, B.d_outA, B.d_outB, B.d_outG);
     e = cudaGetLastError();
     if (e == cudaSuccess && B.precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {
-        batchNearKernel<<<148 * 8, 256, 0, st>>>(B.d_blob, B.d_segs, B.d_points, B.d_outA, B.d_outB, B.d_outG, work,
-                                                 B.work_capacity, B.d_work_count);
+        batchNearListKernel<<<(unsigned)std::min(B.nitems, 148 * 64), 128, 0, st>>>(
+            B.d_blob, B.d_segs, items, B.nitems, B.fields_mask, B.d_points, work, B.work_capacity, B.d_work_count);
+        batchNearKernel<<<148 * 8, 256, 0, st>>>(B.d_blob, B.d_segs, items, B.nitems, B.d_points, B.d_outA, B.d_outB,
+                                                 B.d_outG, work, B.work_capacity, B.d_work_count);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? CCOIL_OK : failMessage(CCOIL_ERR_CUDA, cudaGetErrorString(e));

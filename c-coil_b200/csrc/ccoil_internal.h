@@ -237,6 +237,7 @@ struct BatchLaunch
     const double *d_points;
     double *d_outA, *d_outB, *d_outG;
     int precision;
+    int fields_mask;  // bits 1 << CCOIL_FIELD_A, _B, _G
     int grid;
     void *d_work = nullptr;
     unsigned long long work_capacity = 0;

@@ -48,15 +48,6 @@ __device__ __forceinline__ void integrateSegment32(const unsigned char *seg, con
     }
 }
 
-// FP64 integration of one segment for a pair that did not fit the work list;
-// kept out of line so the FP32 kernel's register budget does not carry it.
-template <int FIELD, int LANES>
-__device__ __noinline__ void integrateSegment64Fallback(const unsigned char *seg, double px, double py, double pz,
-                                                        int lane, double *acc)
-{
-    integrateSegment64<FIELD, LANES>(seg, px, py, pz, lane, acc);
-}
-
 // Near-field work list entry: (point, segment)
 struct NearPair
 {

@@ -89,3 +89,25 @@ def test_more_near_pairs_than_the_list_holds(ccoil):
         assert fn(structs, len(coils), ctypes.c_void_p(x.data_ptr()), n, field, ctypes.c_void_p(out.data_ptr()),
                   ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, L.ccoil_last_error_message()
         assert rel_err(out.cpu().numpy(), want).max() < TOL, field
+
+
+def test_batch_near_pairs_beyond_the_list_and_repeatable(ccoil):
+    # one system whose points all lie in the winding boxes of 12 coils: 4.3 million
+    # pairs over two fields, more than the batch's list; a second, shorter system
+    coils = [ccoil.Coil(0.1, 0.02, 0.05, 10 + i, 1.0 + i) for i in range(12)]
+    g = np.random.default_rng(6)
+
+    def ring(n):
+        r, phi = g.uniform(0.095, 0.125, n), g.uniform(0.0, 2.0 * np.pi, n)
+        return np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, n)], axis=1)
+
+    for systems in ([(coils, ring(180001)), (coils[:5], ring(77))], [(coils, ring(3001)), (coils[3:], ring(1))]):
+        plan = ccoil.BatchPlan(systems, fields=("A", "B"), precision=ccoil.PrecisionMode.FP32_COMPENSATED)
+        first = {f: v.clone() for f, v in plan.run().items()}
+        again = plan.run()
+        for f, field in (("A", 0), ("B", 1)):
+            assert bool((first[f] == again[f]).all()), f
+            for (c, pts), got in zip(systems, plan.split(first[f])):
+                want = ccoil.FieldPlan([k.struct() for k in c], field, ccoil.PrecisionMode.FP32_COMPENSATED)(pts)
+                assert rel_err(got.cpu().numpy(), want).max() < TOL, f
+        plan.close()
