@@ -390,16 +390,10 @@ __device__ __forceinline__ void integrateSegmentRefine(const unsigned char *seg,
 // (FP64 atomics).  The selection lists the pairs segment-major, so the lanes
 // of a warp read one segment's tables and run loops of the same length.
 // Grid-stride over the device-side count.
-// CTAs per SM of the FP64 pair pass: the most at which each field's FP64
-// integrands compile without spills (vector potential 78 registers, field 96,
-// gradient 122)
-#ifndef CCOIL_REFINE_MIN_BLOCKS_B
-#define CCOIL_REFINE_MIN_BLOCKS_B 5
-#endif
-constexpr int refineMinBlocks(int field)
-{
-    return field == CCOIL_FIELD_B ? CCOIL_REFINE_MIN_BLOCKS_B : (field == CCOIL_FIELD_G ? 4 : 6);
-}
+// CTAs per SM of the FP64 pair pass: several nodes in flight per thread without
+// spills (vector potential 120 registers, field 112, gradient 142) measured 1 %
+// faster for the whole call than the most CTAs that fit without (6, 5 and 4)
+constexpr int refineMinBlocks(int field) { return field == CCOIL_FIELD_G ? 3 : 4; }
 template <int FIELD>
 __global__ void __launch_bounds__(128, refineMinBlocks(FIELD)) refinePairsKernel64(
     const unsigned char *__restrict__ blob, const SegmentDesc *__restrict__ segs, const double *__restrict__ points,

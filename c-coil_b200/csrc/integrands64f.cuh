@@ -48,6 +48,11 @@ __device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, double cA
         den = above ? a2 : (below ? a1 : D);
     };
     double part = 0.0;
+    // two mirror pairs in flight in the refinement pass (A of 128 coils at 2^17
+    // points 17.5 -> 17.3 ms with 120 registers); the arrangement kernels call
+    // this within 56 registers
+    constexpr int kUnroll = PAIRED ? 2 : 1;
+#pragma unroll kUnroll
     for (int m = 0; m < n / 2; ++m)
     {
         const double2 q = pt[PAIRED ? 2 * m : m], qm = pt[PAIRED ? 2 * m + 1 : n - 1 - m];
@@ -123,7 +128,7 @@ __device__ __forceinline__ double segmentA64Fast(const SegmentHeader &h, const d
     return sum;
 }
 
-// The field of one segment at one point, one thread:
+// The field of one segment at one point, one thread, four nodes in flight:
 // the reference's node values with every 1/sqrt(D) from rsqrt64 (fast method:
 // w c (g2 - g1) and w (p^2 - p r c) / rho^2 (top g1 - bot g2); slow method:
 // w g^3 (p^2 - p r c) and w g^3 p zl c)
@@ -131,6 +136,7 @@ template <bool CHECKED>
 __device__ __forceinline__ void phiLoopB64(const double2 *pt, int n, double cA, double cB, double cC, double d1,
                                            double d2, double top, double bot, double &h0, double &z0)
 {
+#pragma unroll 4
     for (int k = 0; k < n; ++k)
     {
         const double2 q = pt[k];
