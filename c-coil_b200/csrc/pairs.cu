@@ -468,6 +468,7 @@ __device__ __forceinline__ void transformDerivatives(double yA, double zA, doubl
 #ifndef CCOIL_PAIR32R_MIN_BLOCKS
 #define CCOIL_PAIR32R_MIN_BLOCKS 9
 #endif
+constexpr int pairThreads(int team) { return team > 4 ? 32 * team : 128; }
 constexpr int pairMinBlocks(int qty, bool fp32, bool refine)
 {
     return refine ? CCOIL_PAIR32R_MIN_BLOCKS
@@ -578,8 +579,11 @@ __device__ __noinline__ double2 pairB32(const SegmentHeader &h, const double2 *t
 // (PairSplit).  Each unit's sums go to `partial` and pairReduceKernel adds an
 // arrangement's units in a fixed order.  LANES > 1 (FP64 M, F/T and position gradient): that many
 // lanes share a secondary node and split the primary's angular nodes.
-template <int QTY, bool FP32, bool REFINE = false, int LANES = 1>
-__global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
+//
+// TEAM > 1 (REFINE): that many warps, a whole CTA, share each arrangement's nodes,
+// since the selection needs the primary's total.
+template <int QTY, bool FP32, bool REFINE = false, int LANES = 1, int TEAM = 1>
+__global__ void __launch_bounds__(pairThreads(TEAM), pairMinBlocks(QTY, FP32, REFINE) * 4 / (pairThreads(TEAM) / 32))
     pairKernel64(const unsigned char *__restrict__ blob, const long long *__restrict__ primOffsets, int nprim,
                  const double *__restrict__ primPoses, const double *__restrict__ secPoses, long long count,
                  double *__restrict__ out, unsigned long long *__restrict__ zAxisCount, int stagedBytes,
@@ -588,16 +592,18 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                  double fraction, PairSplit split, double *__restrict__ partial)
 {
     extern __shared__ __align__(16) unsigned char stagedPair[];
-    __shared__ WarpPose warpPoses[4];
-    __shared__ int nearLists[4][64];  // FP32: each warp's deferred near-field secondary nodes
+    constexpr int THREADS = pairThreads(TEAM), WARPS = THREADS / 32;
+    __shared__ WarpPose warpPoses[WARPS];
+    __shared__ int nearLists[WARPS][64];  // FP32: each warp's deferred near-field secondary nodes
     constexpr int W = QTY == 0 ? 1 : QTY == 1 ? 6 : QTY == 2 ? 3 : 14;
     // Running sums in shared memory: each thread's sums over its secondary nodes
     // (one column per thread, so a warp's accesses hit 32 consecutive doubles)
     // and each warp's sums over the primaries (lane 0).  Held in registers they
     // stayed live across the out-of-line quadrature call and spilled to local
     // memory at the register budget of 9 CTAs per SM.
-    __shared__ double laneSums[W][128];
-    __shared__ double warpSums[4][W];
+    __shared__ double laneSums[W][THREADS];
+    __shared__ double warpSums[WARPS][W];
+    __shared__ double teamSums[TEAM > 1 ? WARPS : 1][W];  // each warp's sums of the current primary
     if (stagedBytes > 0)
     {
         const int4 *src = reinterpret_cast<const int4 *>(blob + primOffsets[0]);
@@ -610,14 +616,17 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
     volatile WarpPose &S = warpPoses[threadIdx.x / 32];
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const long long warps = (long long)gridDim.x * blockDim.x / 32;
-    double *part = &laneSums[0][threadIdx.x];  // part[128 i]: this thread's sum i
+    double *part = &laneSums[0][threadIdx.x];  // part[THREADS i]: this thread's sum i
     double *total = warpSums[threadIdx.x / 32];
     const int perArr = split.groups * split.parts;
     const long long units = count * perArr;
-    for (long long u = warp; u < units; u += warps)
+    // a team takes whole arrangements, each warp its part of the nodes
+    const int parts = TEAM > 1 ? TEAM : split.parts;
+    for (long long u = TEAM > 1 ? (long long)blockIdx.x : warp; u < units; u += TEAM > 1 ? (long long)gridDim.x : warps)
     {
         const long long a = u / perArr;
-        const int piece = (int)(u - a * perArr), group = piece / split.parts, part_i = piece - group * split.parts;
+        const int piece = (int)(u - a * perArr), group = piece / split.parts;
+        const int part_i = TEAM > 1 ? threadIdx.x / 32 : piece - group * split.parts;
         const int j0 = (int)((long long)nprim * group / split.groups);
         const int j1 = (int)((long long)nprim * (group + 1) / split.groups);
         if (lane == 0)
@@ -708,11 +717,11 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
             // this unit's secondary nodes: whole warp iterations of 32 / LANES nodes
             constexpr int STEP = 32 / LANES;
             const int nodes = ph.s_nl * ph.s_nt * ph.s_na, iters = (nodes + STEP - 1) / STEP;
-            const int nBegin = (int)((long long)iters * part_i / split.parts) * STEP;
-            const int nsec = min(nodes, (int)((long long)iters * (part_i + 1) / split.parts) * STEP);
+            const int nBegin = (int)((long long)iters * part_i / parts) * STEP;
+            const int nsec = min(nodes, (int)((long long)iters * (part_i + 1) / parts) * STEP);
             const int sub = lane % LANES, slot = lane / LANES;
             for (int i = 0; i < W; ++i)
-                part[128 * i] = 0.0;
+                part[THREADS * i] = 0.0;
             // every lane runs the same number of iterations (warp-uniform choices
             // below); a lane past the end evaluates the last node and drops it
             // One secondary node per lane.  mode 0: the FP64 kernel; mode 1: the FP32
@@ -721,7 +730,9 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
             int nNear = 0;
             int *list = nearLists[threadIdx.x / 32];
             // REFINE: this warp's node contributions
-            double *scr = REFINE ? nodeScratch + (size_t)warp * (size_t)scratchNodes * W : nullptr;
+            double *scr = REFINE ? nodeScratch + (size_t)(TEAM > 1 ? (long long)blockIdx.x : warp) *
+                                                   (size_t)scratchNodes * W
+                                 : nullptr;
             auto node = [&](int n, bool valid, int mode) {
                 const int k = n % ph.s_na, lt_i = n / ph.s_na;
                 const int t = lt_i % ph.s_nt, l = lt_i / ph.s_nt;
@@ -856,7 +867,7 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                     g[13] = gB;
                     if (valid)
                         for (int i = 0; i < 14; ++i)
-                            part[128 * i] += g[i] * w;
+                            part[THREADS * i] += g[i] * w;
                 }
                 else if (QTY == 2)
                 {
@@ -880,7 +891,7 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                         o[i] = S.T[3 * i] * v[0] + S.T[3 * i + 1] * v[1] + S.T[3 * i + 2] * v[2];
                     if (valid)
                         for (int i = 0; i < 3; ++i)
-                            part[128 * i] += o[i] * w;
+                            part[THREADS * i] += o[i] * w;
                 }
                 else
                 {
@@ -910,8 +921,8 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                     if (valid)
                         for (int i = 0; i < 3; ++i)
                         {
-                            part[128 * i] += dF[i];
-                            part[128 * (3 + i)] += dT[i];
+                            part[THREADS * i] += dF[i];
+                            part[THREADS * (3 + i)] += dT[i];
                             if (REFINE && far)
                             {
                                 scr[(size_t)n * W + i] = dF[i];
@@ -957,21 +968,35 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
             {
                 // the primary's totals (every lane), then the dominating nodes in FP64;
                 // node n was evaluated, and its contribution stored, by lane n % 32
+                if (TEAM > 1)
+                {
+                    for (int i = 0; i < W; ++i)
+                    {
+                        const double v = laneSum<32>(part[THREADS * i]);
+                        if (lane == 0)
+                            teamSums[TEAM > 1 ? threadIdx.x / 32 : 0][i] = v;
+                    }
+                    __syncthreads();
+                }
                 double lim[2] = {0.0, 0.0};
                 for (int g = 0; g < (QTY == 0 ? 1 : 2); ++g)
                 {
                     double n2 = 0.0;
                     for (int i = 0; i < (QTY == 0 ? 1 : 3); ++i)
                     {
-                        double v = part[128 * (3 * g + i)];
-#pragma unroll
-                        for (int off = 16; off > 0; off /= 2)
-                            v += __shfl_xor_sync(0xffffffffu, v, off);
+                        double v = 0.0;
+                        if (TEAM > 1)
+                            for (int t = 0; t < TEAM; ++t)
+                                v += teamSums[TEAM > 1 ? t : 0][3 * g + i];
+                        else
+                            v = laneSum<32>(part[THREADS * (3 * g + i)]);
                         n2 += v * v;
                     }
                     lim[g] = fraction * fraction * n2;  // not finite: nothing is picked
                 }
-                for (int b0 = 0; b0 < nsec; b0 += 32)
+                if (TEAM > 1)
+                    __syncthreads();  // every warp has read the totals
+                for (int b0 = nBegin; b0 < nsec; b0 += 32)
                 {
                     const int n = b0 + lane;
                     bool pick = false;
@@ -987,7 +1012,7 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                                    c[3] * c[3] + c[4] * c[4] + c[5] * c[5] > lim[1];
                         if (pick)
                             for (int i = 0; i < W; ++i)
-                                part[128 * i] -= c[i];
+                                part[THREADS * i] -= c[i];
                     }
                     const unsigned bal = __ballot_sync(0xffffffffu, pick);
                     if (pick)
@@ -1003,7 +1028,7 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
 #pragma unroll
             for (int i = 0; i < W; ++i)
             {
-                double v = part[128 * i];
+                double v = part[THREADS * i];
 #pragma unroll
                 for (int off = 16; off > 0; off /= 2)
                     v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -1011,7 +1036,17 @@ __global__ void __launch_bounds__(128, pairMinBlocks(QTY, FP32, REFINE))
                     total[i] += v * scale;
             }
         }
-        if (lane == 0)
+        if (TEAM > 1)
+        {
+            // warp 0 adds the warps' sums, in order
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int t = 1; t < TEAM; ++t)
+                    for (int i = 0; i < W; ++i)
+                        total[i] += warpSums[TEAM > 1 ? t : 0][i];
+            __syncthreads();
+        }
+        if (lane == 0 && (TEAM == 1 || threadIdx.x == 0))
         {
             double *dst = partial ? partial + W * u : out + W * a;
 #pragma unroll
@@ -1445,6 +1480,12 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
             lanes = 8;
         split = pairSplit(count, primary_count, secNodes, 32 / lanes, resident);
     }
+    // the refining kernel shares few arrangements among the warps of a CTA: 12 while
+    // every arrangement then has a resident CTA, else 4 up to three waves of whole
+    // arrangements (M of 1, 444, 2,000, 8,000 and 32,768 arrangements with one warp
+    // each 0.40, 1.33, 1.73, 2.95 and 9.4 ms, with 4 or 12 0.11, 0.44, 0.93, 2.69 and
+    // 9.9: each warp's last FP64 batch of 32 nodes is partly empty)
+    const int team = !refine ? 1 : count <= 148LL * 3 ? 12 : count <= resident * 3 ? 4 : 1;
     const long long perArr = (long long)split.groups * split.parts;
     if (perArr > 1)
     {
@@ -1452,7 +1493,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         if (e != cudaSuccess)
             return cudaFail(e, "arrangement partial sums");
     }
-    long long blocks = (count * perArr + 3) / 4;
+    long long blocks = team > 1 ? count : (count * perArr + 3) / 4;
     if (blocks > 148LL * 64)
         blocks = 148LL * 64;
     // FP32_REFINED: every warp's region of node contributions (the grid strides over
@@ -1462,7 +1503,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     {
         // at most kPairRefineScratchBytes: a secondary with many nodes runs on fewer
         // warps (each keeps 1 or 6 doubles per node), never fewer than one CTA per SM
-        const size_t perBlock = sizeof(double) * (size_t)width * (size_t)scratchNodes * 4;
+        const size_t perBlock = sizeof(double) * (size_t)width * (size_t)scratchNodes * (team > 1 ? 1 : 4);
         const long long fit = (long long)(kPairRefineScratchBytes / perBlock);
         blocks = std::max(1LL, std::min(blocks, std::max(fit, 148LL)));
         e = dScratch.alloc(perBlock * (size_t)blocks, st);
@@ -1480,7 +1521,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     auto *zL = static_cast<long long *>(dZList.p);
     auto *zN = static_cast<unsigned long long *>(dZCount.p);
 #define CCOIL_PAIR_LAUNCH(Q, F, ...)                                                                                   \
-    pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, 128, smem, st>>>(                                          \
+    pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, pairThreads(team), smem, st>>>(                                          \
         dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction,  \
         split, partial)
     if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32 && lanes == 8)
@@ -1491,6 +1532,14 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         CCOIL_PAIR_LAUNCH(2, false, false, 8);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32)
         CCOIL_PAIR_LAUNCH(0, false);
+    else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && refine && team == 12)
+        CCOIL_PAIR_LAUNCH(0, true, true, 1, 12);
+    else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && refine && team == 4)
+        CCOIL_PAIR_LAUNCH(0, true, true, 1, 4);
+    else if (quantity == CCOIL_PAIR_FORCE_TORQUE && refine && team == 12)
+        CCOIL_PAIR_LAUNCH(1, true, true, 1, 12);
+    else if (quantity == CCOIL_PAIR_FORCE_TORQUE && refine && team == 4)
+        CCOIL_PAIR_LAUNCH(1, true, true, 1, 4);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && refine)
         CCOIL_PAIR_LAUNCH(0, true, true);
     else if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE)
