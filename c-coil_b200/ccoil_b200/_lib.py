@@ -59,6 +59,10 @@ class CCoilError(RuntimeError):
 _lib = None
 
 
+class PoseArraysStruct(ctypes.Structure):
+    _fields_ = [("position", ctypes.c_void_p), ("y_angle", ctypes.c_void_p), ("z_angle", ctypes.c_void_p)]
+
+
 def lib():
     """Load the library once; raises if it has not been built."""
     global _lib
@@ -107,6 +111,10 @@ def lib():
     L.ccoil_pair_arrangements_zaxis.argtypes = [cp, ctypes.c_int, cp, pp, pp, vp, vp, ctypes.c_longlong,
                                                 ctypes.c_int, ctypes.c_int, vp, ctypes.POINTER(ctypes.c_longlong),
                                                 ctypes.c_int, vp]
+    L.ccoil_pair_arrangements_arrays.argtypes = [cp, ctypes.c_int, cp, pp, pp, ctypes.POINTER(PoseArraysStruct),
+                                                 ctypes.POINTER(PoseArraysStruct), ctypes.c_longlong, ctypes.c_int,
+                                                 ctypes.c_int, vp, ctypes.POINTER(ctypes.c_longlong), vp]
+    L.ccoil_coils_from_params.argtypes = [dp, pp, ctypes.c_int, cp]
     _lib = L
     return L
 

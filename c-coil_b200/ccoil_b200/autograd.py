@@ -39,15 +39,8 @@ from .coil import Coil, PrecisionArguments, PrecisionFactor, PrecisionMode, _fac
 PARAMS = ("R", "a", "b", "NI", "x", "y", "z", "y_angle", "z_angle")
 
 
-def _structs(params, precisions):
-    out = []
-    for q, pa in zip(params, precisions):
-        s = _lib.CoilStruct()
-        pos = (ctypes.c_double * 3)(q[4], q[5], q[6])
-        check(lib().ccoil_coil_init(q[0], q[1], q[2], 1, q[3], 0.0, pos, q[7], q[8], 5.0, 0, ctypes.byref(s)))
-        s.precision = pa.to_struct()
-        out.append(s)
-    return out
+def _precision_array(precisions):
+    return (_lib.PrecisionArgsStruct * max(len(precisions), 1))(*[p.to_struct() for p in precisions])
 
 
 def precisions_for(params, precision_factor=5.0):
@@ -63,28 +56,28 @@ def precisions_for(params, precision_factor=5.0):
 class _BField(torch.autograd.Function):
     @staticmethod
     def forward(ctx, params, points, precisions):
-        q = params.detach().to("cpu", torch.float64).numpy()
-        structs = _structs(q, precisions)
+        q = np.array(params.detach().to("cpu", torch.float64).numpy(), order="C")
+        n = q.shape[0]
+        precs = _precision_array(precisions)
+        arr = (_lib.CoilStruct * max(n, 1))()
+        check(lib().ccoil_coils_from_params(q.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), precs, n, arr))
         pts = points.detach().to(torch.float64).contiguous()
         mode = PrecisionMode.FP32_COMPENSATED if points.dtype == torch.float32 else PrecisionMode.FP64
         out = torch.empty((pts.shape[0], 3), dtype=torch.float64, device=pts.device)
-        arr = (_lib.CoilStruct * max(len(structs), 1))(*structs)
         st = torch.cuda.current_stream(pts.device).cuda_stream
-        check(lib().ccoil_compute_fields(arr, len(structs), ctypes.c_void_p(pts.data_ptr()), pts.shape[0],
+        check(lib().ccoil_compute_fields(arr, n, ctypes.c_void_p(pts.data_ptr()), pts.shape[0],
                                          _lib.FIELD_B, int(mode), ctypes.c_void_p(out.data_ptr()),
                                          _lib.MEMORY_DEVICE, ctypes.c_void_p(st)))
         ctx.save_for_backward(params, pts)
-        ctx.precisions = precisions
-        ctx.points_dtype = points.dtype
+        ctx.q, ctx.precs = q, precs  # the parameters' values and precisions as the native calls take them
         return out.to(points.dtype)
 
     @staticmethod
     def backward(ctx, grad_b):
         params, pts = ctx.saved_tensors
-        q = np.ascontiguousarray(params.detach().to("cpu", torch.float64).numpy())
+        q, precs = ctx.q, ctx.precs
         g = grad_b.detach().to(torch.float64).contiguous()
         gp = torch.zeros((q.shape[0], 9), dtype=torch.float64, device=pts.device)
-        precs = (_lib.PrecisionArgsStruct * max(len(ctx.precisions), 1))(*[p.to_struct() for p in ctx.precisions])
         st = torch.cuda.current_stream(pts.device).cuda_stream
         check(lib().ccoil_b_field_adjoint(q.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), precs, q.shape[0],
                                           ctypes.c_void_p(pts.data_ptr()), pts.shape[0],
@@ -134,41 +127,56 @@ def _pair_structs(g1, g2, pp, sp):
     return s1, s2
 
 
+def _to_host(a, b):
+    """Two small tensors as float64 numpy arrays, in one copy where they share a device."""
+    a, b = a.detach(), b.detach()
+    if a.is_cuda and a.device == b.device and a.shape == b.shape:
+        return torch.stack([a.to(torch.float64), b.to(torch.float64)]).cpu().numpy()
+    return tuple(v.to("cpu", torch.float64).numpy() for v in (a, b))
+
+
 class _MutualInductance(torch.autograd.Function):
     @staticmethod
     def forward(ctx, geom1, geom2, poses1, poses2, precisions):
-        from .coil import _pair_arrangements
-        g1 = geom1.detach().to("cpu", torch.float64).numpy()
-        g2 = geom2.detach().to("cpu", torch.float64).numpy()
-        p1 = np.ascontiguousarray(poses1.detach().to("cpu", torch.float64).numpy())
-        p2 = np.ascontiguousarray(poses2.detach().to("cpu", torch.float64).numpy())
-        if p1.shape != p2.shape or p1.ndim != 2 or p1.shape[1] != 5:
+        from .coil import _pair_arrangements, pair_arrangements_device
+        g1, g2 = _to_host(geom1, geom2)
+        if poses1.shape != poses2.shape or poses1.ndim != 2 or poses1.shape[1] != 5:
             raise ValueError("poses must be (n, 5) arrays of equal shape")
         pp, sp = precisions
         s1, s2 = _pair_structs(g1, g2, pp, sp)
         # float32 poses: the primary's quadrature in FP32 (FP64 near its winding and in the sums)
         mode = PrecisionMode.FP32_COMPENSATED if poses2.dtype == torch.float32 else PrecisionMode.FP64
-        out, _ = _pair_arrangements([s1], s2, [sp.to_struct()], p1, p2,
-                                    _lib.PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT, precision_mode=mode)
+        quantity = _lib.PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT
+        if poses1.is_cuda and poses1.device == poses2.device and poses1.device.index == torch.cuda.current_device():
+            # poses on the current GPU: results and, in the backward pass, gradients stay there
+            p1, p2 = (p.detach().to(torch.float64).contiguous() for p in (poses1, poses2))
+            out = torch.empty((p2.shape[0], 14), dtype=torch.float64, device=p2.device)
+            st = torch.cuda.current_stream(p2.device).cuda_stream
+            pair_arrangements_device([s1], s2, [sp.to_struct()], p1, p2, quantity, out, st, mode)
+        else:
+            p1, p2 = (np.ascontiguousarray(p.detach().to("cpu", torch.float64).numpy()) for p in (poses1, poses2))
+            out = torch.from_numpy(_pair_arrangements([s1], s2, [sp.to_struct()], p1, p2, quantity,
+                                                      precision_mode=mode)[0])
         out = out * (g1[3] * g2[3])
         ctx.out = out
         ctx.turns = (g1[3], g2[3])
         ctx.devices = (geom1.device, geom2.device, poses1.device, poses2.device)
         ctx.dtypes = (geom1.dtype, geom2.dtype, poses1.dtype, poses2.dtype)
-        return torch.from_numpy(out[:, 0].copy()).to(poses2.device, poses2.dtype)
+        return out[:, 0].clone().to(poses2.device, poses2.dtype)
 
     @staticmethod
     def backward(ctx, grad_m):
         out = ctx.out
         n1, n2 = ctx.turns
-        g = grad_m.detach().to("cpu", torch.float64).numpy()
-        M = out[:, 0]
-        d1 = np.array([g @ out[:, 1], g @ out[:, 2], g @ out[:, 3], g @ M / n1])
-        d2 = np.array([g @ out[:, 6], g @ out[:, 7], g @ out[:, 8], g @ M / n2])
-        dp2 = np.concatenate([out[:, 9:12], out[:, 12:14]], axis=1) * g[:, None]
-        dp1 = np.concatenate([-out[:, 9:12], out[:, 4:6]], axis=1) * g[:, None]
-        res = [torch.from_numpy(v).to(dev, dt) for v, dev, dt in zip((d1, d2, dp1, dp2), ctx.devices, ctx.dtypes)]
-        return res[0], res[1], res[2], res[3], None
+        g = grad_m.detach().to(out.device, torch.float64)
+        weighted = out * g[:, None]
+        s = weighted.sum(0)
+        d1 = torch.stack([s[1], s[2], s[3], s[0] / n1])
+        d2 = torch.stack([s[6], s[7], s[8], s[0] / n2])
+        dp2 = weighted[:, 9:14]
+        dp1 = torch.cat([-weighted[:, 9:12], weighted[:, 4:6]], dim=1)
+        res = [v.to(dev, dt) for v, dev, dt in zip((d1, d2, dp1, dp2), ctx.devices, ctx.dtypes)]
+        return res[0], res[1], res[2], res[3].contiguous(), None
 
 
 def mutual_inductance(geom1, geom2, poses1, poses2, precisions=None, precision_factor=5.0):

@@ -139,12 +139,31 @@ def _points_host(points):
 
 
 def _evaluate(coil_structs, points, field, precision, lanes=0, stream=None):
-    """Runs one field evaluation through a temporary plan."""
-    plan = FieldPlan(coil_structs, field, precision)
-    try:
-        return plan(points, lanes=lanes, stream=stream)
-    finally:
-        plan.close()
+    """Runs one field evaluation: in one call, or through a temporary plan for a lane count."""
+    if lanes:
+        plan = FieldPlan(coil_structs, field, precision)
+        try:
+            return plan(points, lanes=lanes, stream=stream)
+        finally:
+            plan.close()
+    n = len(coil_structs)
+    arr = (_lib.CoilStruct * max(n, 1))(*coil_structs)
+    width = 9 if int(field) == _lib.FIELD_G else 3
+    if _is_torch_cuda(points):
+        import torch
+        pts = points.contiguous().to(torch.float64)
+        if pts.ndim != 2 or pts.shape[1] != 3:
+            raise ValueError("points must have shape (n, 3)")
+        out = torch.empty((pts.shape[0], width), dtype=torch.float64, device=pts.device)
+        st = stream if stream is not None else torch.cuda.current_stream(pts.device).cuda_stream
+        check(lib().ccoil_compute_fields(arr, n, pts.data_ptr(), pts.shape[0], int(field), int(precision),
+                                         out.data_ptr(), _lib.MEMORY_DEVICE, st))
+        return out
+    pts = _points_host(points)
+    out = np.empty((pts.shape[0], width), dtype=np.float64)
+    check(lib().ccoil_compute_fields(arr, n, pts.ctypes.data, pts.shape[0], int(field), int(precision),
+                                     out.ctypes.data, _lib.MEMORY_HOST, stream or 0))
+    return out
 
 
 class FieldPlan:
@@ -210,38 +229,52 @@ def _shape(res, field):
     return res
 
 
+class _PoseArrays:
+    """Poses as the three contiguous float64 arrays the native call takes."""
+
+    def __init__(self, positions, y_angles, z_angles):
+        self.position = np.ascontiguousarray(positions, dtype=np.float64).reshape(-1, 3)
+        self.y = np.ascontiguousarray(y_angles, dtype=np.float64).reshape(-1)
+        self.z = np.ascontiguousarray(z_angles, dtype=np.float64).reshape(-1)
+        if not (len(self.position) == len(self.y) == len(self.z)):
+            raise ValueError("Array sizes do not match!")
+        self.struct = _lib.PoseArraysStruct(self.position.ctypes.data, self.y.ctypes.data, self.z.ctypes.data)
+
+    def __len__(self):
+        return len(self.y)
+
+
 def _poses(positions, y_angles, z_angles):
-    pos = np.ascontiguousarray(positions, dtype=np.float64).reshape(-1, 3)
-    y = np.ascontiguousarray(y_angles, dtype=np.float64).reshape(-1)
-    z = np.ascontiguousarray(z_angles, dtype=np.float64).reshape(-1)
-    if not (len(pos) == len(y) == len(z)):
-        raise ValueError("Array sizes do not match!")
-    return np.ascontiguousarray(np.concatenate([pos, y[:, None], z[:, None]], axis=1))
+    """Packed (n, 5) poses."""
+    p = _PoseArrays(positions, y_angles, z_angles)
+    return np.ascontiguousarray(np.concatenate([p.position, p.y[:, None], p.z[:, None]], axis=1))
 
 
 def _pair_arrangements(primaries, secondary, sec_precisions, primary_poses, secondary_poses, quantity,
                        precision_mode=PrecisionMode.FP64, zaxis_precisions=None):
-    """Runs ccoil_pair_arrangements (ccoil_pair_arrangements_zaxis when z-axis pair arguments
-    [primary, secondary] per primary are given); returns (values, number of exact z-axis pairs)."""
+    """Runs ccoil_pair_arrangements_zaxis (without z-axis pair arguments [primary, secondary] per primary:
+    ccoil_pair_arrangements) on packed (n, 5) poses, or ccoil_pair_arrangements_arrays on _PoseArrays;
+    returns (values, number of exact z-axis pairs)."""
     n = len(secondary_poses)
     width = {_lib.PAIR_MUTUAL_INDUCTANCE: 1, _lib.PAIR_FORCE_TORQUE: 6,
              _lib.PAIR_MUTUAL_INDUCTANCE_GRADIENT: 3, _lib.PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT: 14}[quantity]
-    out = np.zeros((n, width))
+    out = np.empty((n, width))
     prim = (_lib.CoilStruct * max(len(primaries), 1))(*primaries)
     secp = (_lib.PrecisionArgsStruct * max(len(sec_precisions), 1))(*sec_precisions)
     zc = ctypes.c_longlong(0)
-    pposes = None if primary_poses is None else primary_poses.ctypes.data_as(ctypes.c_void_p)
-    if zaxis_precisions is None:
-        check(lib().ccoil_pair_arrangements(
-            prim, len(primaries), ctypes.byref(secondary), secp, pposes,
-            secondary_poses.ctypes.data_as(ctypes.c_void_p), n, quantity, int(precision_mode),
-            out.ctypes.data_as(ctypes.c_void_p), ctypes.byref(zc), _lib.MEMORY_HOST, None))
+    zp = None if zaxis_precisions is None else (
+        _lib.PrecisionArgsStruct * max(len(zaxis_precisions), 1))(*zaxis_precisions)
+    if isinstance(secondary_poses, _PoseArrays):
+        check(lib().ccoil_pair_arrangements_arrays(
+            prim, len(primaries), ctypes.byref(secondary), secp, zp,
+            None if primary_poses is None else ctypes.byref(primary_poses.struct),
+            ctypes.byref(secondary_poses.struct), n, quantity, int(precision_mode), out.ctypes.data,
+            ctypes.byref(zc), None))
     else:
-        zp = (_lib.PrecisionArgsStruct * max(len(zaxis_precisions), 1))(*zaxis_precisions)
         check(lib().ccoil_pair_arrangements_zaxis(
-            prim, len(primaries), ctypes.byref(secondary), secp, zp, pposes,
-            secondary_poses.ctypes.data_as(ctypes.c_void_p), n, quantity, int(precision_mode),
-            out.ctypes.data_as(ctypes.c_void_p), ctypes.byref(zc), _lib.MEMORY_HOST, None))
+            prim, len(primaries), ctypes.byref(secondary), secp, zp,
+            None if primary_poses is None else primary_poses.ctypes.data, secondary_poses.ctypes.data, n, quantity,
+            int(precision_mode), out.ctypes.data, ctypes.byref(zc), _lib.MEMORY_HOST, None))
     return (out[:, 0] if width == 1 else out), zc.value
 
 
@@ -375,8 +408,8 @@ class Coil:
         if ComputeMethod(compute_method) != ComputeMethod.GPU:
             raise NotImplementedError("this package provides the ComputeMethod.GPU path only")
         pp, sp = Coil._pair_args(primary, secondary, _factor(precision_factor))
-        ppose = _poses(primary_positions, primary_y_angles, primary_z_angles)
-        spose = _poses(secondary_positions, secondary_y_angles, secondary_z_angles)
+        ppose = _PoseArrays(primary_positions, primary_y_angles, primary_z_angles)
+        spose = _PoseArrays(secondary_positions, secondary_y_angles, secondary_z_angles)
         if len(ppose) != len(spose):
             raise ValueError("Array sizes do not match!")
         zargs = None
@@ -575,7 +608,7 @@ class CoilGroup:
             za = CoilPairArguments.get_appropriate_coil_pair_arguments(m, secondary, pf, ComputeMethod.CPU_ST,
                                                                        z_axis_case=True)
             zargs += [za.primary_precision.to_struct(), za.secondary_precision.to_struct()]
-        spose = _poses(positions, y_angles, z_angles)
+        spose = _PoseArrays(positions, y_angles, z_angles)
         vals, _ = _pair_arrangements(prims, secondary.struct(), secs, None, spose, quantity, precision_mode,
                                      zargs if quantity in (_lib.PAIR_MUTUAL_INDUCTANCE, _lib.PAIR_FORCE_TORQUE)
                                      else None)

@@ -21,20 +21,24 @@ namespace
 // never allocates)
 thread_local char t_error[512] = "";
 
-// Grow-only device buffer owned by a plan.
+// Grow-only device buffer owned by a plan.  A plan that a user keeps serves any
+// stream, so its buffers are allocated and replaced with the device idle; the plan
+// of a one-shot call (scoped) has its buffers in the order of the call's stream.
+struct BufferOwner
+{
+    bool scoped = false;
+    cudaStream_t stream = nullptr;
+};
 struct DeviceBuffer
 {
     void *ptr = nullptr;
     size_t bytes = 0;
-    int reserve(size_t n);
-    void release()
+    int reserve(size_t n, const BufferOwner &o);
+    // the device is idle, or the owner is scoped
+    void release(const BufferOwner &o)
     {
         if (ptr)
-        {
-            cudaDeviceSynchronize();
-            cudaFreeAsync(ptr, nullptr);
-            cudaStreamSynchronize(nullptr);
-        }
+            cudaFreeAsync(ptr, o.scoped ? o.stream : nullptr);
         ptr = nullptr;
         bytes = 0;
     }
@@ -118,16 +122,16 @@ cudaError_t scratchAlloc(void **p, size_t bytes, cudaStream_t st)
 
 namespace
 {
-// plan buffers: allocated and released in the order of the legacy default
-// stream, which waits for all blocking streams; release waits for the device
-// so that no kernel on any stream still reads the buffer
-int DeviceBuffer::reserve(size_t n)
+int DeviceBuffer::reserve(size_t n, const BufferOwner &o)
 {
     if (n <= bytes)
         return CCOIL_OK;
-    release();
-    cudaError_t e = scratchAlloc(&ptr, n, nullptr);
-    if (e == cudaSuccess)
+    // no kernel on any stream may still read a buffer that is replaced
+    if (ptr && !o.scoped)
+        cudaDeviceSynchronize();
+    release(o);
+    cudaError_t e = scratchAlloc(&ptr, n, o.scoped ? o.stream : nullptr);
+    if (e == cudaSuccess && !o.scoped)
         e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess)
     {
@@ -186,6 +190,10 @@ FieldSplit fieldSplit(long long npts, int lanes, int nseg, int thickness, long l
     return s;
 }
 
+// host arrays up to this size are packed into one copy with a call's tables: a
+// copy costs ~4 us whatever its size below that
+constexpr size_t kPackedCopyBytes = size_t(1) << 16;
+
 bool validLanes(int l) { return l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32; }
 } // namespace
 } // namespace ccoil
@@ -199,74 +207,20 @@ struct ccoil_field_plan
     int coil_count = 0;
     int thickness = 1;    // most thickness nodes of a segment
     long long nodes = 0;  // quadrature nodes of all segments
-    SegmentSet set;
-    DeviceBuffer blob, segs, points, out, work, workCount;
+    SegmentSet set;       // set.blob holds the blobs and, after them, the descriptors
+    size_t segsOffset = 0;
+    BufferOwner owner;
+    DeviceBuffer tables, points, out, work, workCount;
     DeviceBuffer contrib, refineSegs, refinedTotal;  // FP32_REFINED
     DeviceBuffer orderScratch, order, sortedPoints, sortedOut;  // point ordering
 };
 
-extern "C" {
-
-int ccoil_abi_version(void) { return CCOIL_ABI_VERSION; }
-
-const char *ccoil_last_error_message(void) { return t_error; }
-
-int ccoil_coil_init(double inner_radius, double thickness, double length, int num_turns, double current,
-                    double sine_frequency, const double position[3], double y_axis_angle, double z_axis_angle,
-                    double precision_factor, int gpu_increments, ccoil_coil_t *out)
+namespace
 {
-    if (!out)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "out is null");
-    if (!(inner_radius > 0.0) || thickness < 0.0 || length < 0.0 || num_turns < 1 || gpu_increments < 0 ||
-        gpu_increments > kMaxOrder)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT,
-                    "coil needs inner_radius > 0, thickness >= 0, length >= 0, num_turns >= 1, "
-                    "gpu_increments in [0, 100]");
-    initCoil(inner_radius, thickness, length, num_turns, current, sine_frequency, position, y_axis_angle,
-             z_axis_angle, *out);
-    out->precision = coilPrecision(*out, precision_factor, gpu_increments);
-    return CCOIL_OK;
-}
-
-int ccoil_precision_arguments(const ccoil_coil_t *coil, double precision_factor, int gpu_increments,
-                              ccoil_precision_args_t *out)
+// Argument checks and the host side of a plan: segment blobs and descriptors in
+// one block, one upload.
+int buildTables(ccoil_field_plan &p, const ccoil_coil_t *coils, int coil_count, int field, int precision)
 {
-    if (!coil || !out)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "null argument");
-    if (gpu_increments < 0 || gpu_increments > kMaxOrder)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "gpu_increments must be in [0, 100]");
-    *out = coilPrecision(*coil, precision_factor, gpu_increments);
-    return CCOIL_OK;
-}
-
-int ccoil_pair_arguments(const ccoil_coil_t *primary, const ccoil_coil_t *secondary, double precision_factor,
-                         int gpu_increments, int z_axis_case, int pure_gpu, ccoil_precision_args_t *primary_out,
-                         ccoil_precision_args_t *secondary_out)
-{
-    if (!primary || !secondary || !primary_out || !secondary_out)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "null argument");
-    if (gpu_increments < 0 || gpu_increments > kMaxOrder)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "gpu_increments must be in [0, 100]");
-    pairPrecision(*primary, *secondary, precision_factor, gpu_increments, z_axis_case != 0, pure_gpu != 0,
-                  *primary_out, *secondary_out);
-    return CCOIL_OK;
-}
-
-int ccoil_legendre(int order, double *nodes, double *weights)
-{
-    if (order < 1 || order > kMaxOrder || !nodes || !weights)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "order must be in [1, 100] and buffers non-null");
-    std::memcpy(nodes, legendreNodes(order), sizeof(double) * order);
-    std::memcpy(weights, legendreWeights(order), sizeof(double) * order);
-    return CCOIL_OK;
-}
-
-int ccoil_field_plan_create(const ccoil_coil_t *coils, int coil_count, int field, int precision,
-                            ccoil_field_plan_t **plan)
-{
-    if (!plan)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "plan is null");
-    *plan = nullptr;
     if (coil_count < 0 || (coil_count > 0 && !coils))
         return fail(CCOIL_ERR_INVALID_ARGUMENT, "coil_count < 0 or coils null");
     if (field < CCOIL_FIELD_A || field > CCOIL_FIELD_G)
@@ -274,91 +228,68 @@ int ccoil_field_plan_create(const ccoil_coil_t *coils, int coil_count, int field
     if (precision != CCOIL_PRECISION_FP64 && precision != CCOIL_PRECISION_FP32_COMPENSATED &&
         precision != CCOIL_PRECISION_FP32_REFINED)
         return fail(CCOIL_ERR_INVALID_ARGUMENT, "precision must be FP64, FP32_COMPENSATED or FP32_REFINED");
-
-    ccoil_field_plan *p = new (std::nothrow) ccoil_field_plan();
-    if (!p)
-        return fail(CCOIL_ERR_OUT_OF_MEMORY, "host allocation failed");
-    p->field = field;
-    p->precision = precision;
-    p->coil_count = coil_count;
+    p.field = field;
+    p.precision = precision;
+    p.coil_count = coil_count;
     std::string err;
     const int tables = precision == CCOIL_PRECISION_FP64 ? CCOIL_PRECISION_FP64 : CCOIL_PRECISION_FP32_COMPENSATED;
-    if (!buildFieldSegments(coils, coil_count, field, tables, p->set, err))
-    {
-        delete p;
+    if (!buildFieldSegments(coils, coil_count, field, tables, p.set, err))
         return fail(CCOIL_ERR_INVALID_ARGUMENT, err);
-    }
-    for (const SegmentDesc &d : p->set.segs)
+    for (const SegmentDesc &d : p.set.segs)
     {
-        const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(p->set.blob.data() + d.offset);
-        p->thickness = std::max(p->thickness, h.n_t);
-        p->nodes += (long long)h.n_t * h.n_phi * std::max(h.n_l, 1);
+        const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(p.set.blob.data() + d.offset);
+        p.thickness = std::max(p.thickness, h.n_t);
+        p.nodes += (long long)h.n_t * h.n_phi * std::max(h.n_l, 1);
     }
-    if (!p->set.segs.empty())
-    {
-        int rc = p->blob.reserve(p->set.blob.size());
-        if (rc == CCOIL_OK)
-            rc = p->segs.reserve(sizeof(SegmentDesc) * p->set.segs.size());
-        if (rc != CCOIL_OK)
-        {
-            ccoil_field_plan_destroy(p);
-            return rc;
-        }
-        cudaError_t e = cudaMemcpy(p->blob.ptr, p->set.blob.data(), p->set.blob.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(p->segs.ptr, p->set.segs.data(), sizeof(SegmentDesc) * p->set.segs.size(),
-                           cudaMemcpyHostToDevice);
-        if (e != cudaSuccess)
-        {
-            ccoil_field_plan_destroy(p);
-            return cudaFail(e, "cudaMemcpy");
-        }
-    }
-    *plan = p;
+    p.segsOffset = p.set.blob.size();  // a multiple of 16
+    const auto *d = reinterpret_cast<const unsigned char *>(p.set.segs.data());
+    p.set.blob.insert(p.set.blob.end(), d, d + sizeof(SegmentDesc) * p.set.segs.size());
     return CCOIL_OK;
 }
 
-int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, long long point_count, double *out,
-                             int memory, int lanes_per_point, void *stream)
+int checkExecute(const double *points, long long point_count, const double *out, int memory)
 {
-    if (!plan)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "plan is null");
     if (point_count < 0 || (point_count > 0 && (!points || !out)))
         return fail(CCOIL_ERR_INVALID_ARGUMENT, "point_count < 0 or null points/out");
     if (memory != CCOIL_MEMORY_HOST && memory != CCOIL_MEMORY_DEVICE)
         return fail(CCOIL_ERR_INVALID_ARGUMENT, "memory must be HOST or DEVICE");
-    if (lanes_per_point != 0 && !validLanes(lanes_per_point))
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "lanes_per_point must be 0, 1, 2, 4, 8, 16 or 32");
-    if (point_count == 0)
-        return CCOIL_OK;
-    // grid.x limit: 2^31-1 CTAs of 128/lanes points
-    if (point_count > (1LL << 36))
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "point_count above 2^36");
+    return CCOIL_OK;
+}
 
+// host results: the copy back, and the wait for it
+int finishHost(double *out, const double *dOut, size_t outBytes, cudaStream_t st)
+{
+    cudaError_t e = cudaMemcpyAsync(out, dOut, outBytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess)
+        return cudaFail(e, "field evaluation");
+    if (!fieldKernelsWait())
+        return CCOIL_OK;
+    long long timeouts = 0;
+    const int rc = readTimeouts(timeouts);
+    if (rc != CCOIL_OK)
+        return rc;
+    if (timeouts > g_timeoutsReported.load())
+    {
+        g_timeoutsReported.store(timeouts);
+        return fail(CCOIL_ERR_TIMEOUT, "a staging wait in the field kernel timed out");
+    }
+    return CCOIL_OK;
+}
+
+// The kernels of one execution, asynchronous on the stream: dPoints and dOut are
+// device memory.
+int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_count, double *dOut, int lanes_per_point,
+              void *stream)
+{
     const int width = plan->field == CCOIL_FIELD_G ? 9 : 3;
     const size_t inBytes = sizeof(double) * 3 * (size_t)point_count;
     const size_t outBytes = sizeof(double) * width * (size_t)point_count;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-
-    const double *dPoints = points;
-    double *dOut = out;
-    if (memory == CCOIL_MEMORY_HOST)
-    {
-        int rc = plan->points.reserve(inBytes);
-        if (rc == CCOIL_OK)
-            rc = plan->out.reserve(outBytes);
-        if (rc != CCOIL_OK)
-            return rc;
-        cudaError_t e = cudaMemcpyAsync(plan->points.ptr, points, inBytes, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess)
-            return cudaFail(e, "host->device copy of points");
-        dPoints = static_cast<const double *>(plan->points.ptr);
-        dOut = static_cast<double *>(plan->out.ptr);
-    }
-
     FieldLaunch L;
-    L.d_blob = static_cast<const unsigned char *>(plan->blob.ptr);
-    L.d_segs = static_cast<const SegmentDesc *>(plan->segs.ptr);
+    L.d_blob = static_cast<const unsigned char *>(plan->tables.ptr);
+    L.d_segs = reinterpret_cast<const SegmentDesc *>(L.d_blob + plan->segsOffset);
     L.nseg = (int)plan->set.segs.size();
     L.d_points = dPoints;
     L.npts = point_count;
@@ -395,9 +326,9 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
         unsigned long long cap = want < limit ? want : limit;
         if (cap == 0)
             cap = 1;
-        int rc0 = plan->work.reserve(cap * kNearPairBytes);
+        int rc0 = plan->work.reserve(cap * kNearPairBytes, plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->workCount.reserve(sizeof(unsigned long long));
+            rc0 = plan->workCount.reserve(sizeof(unsigned long long), plan->owner);
         if (rc0 != CCOIL_OK)
             return rc0;
         L.d_work = plan->work.ptr;
@@ -407,11 +338,11 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
     }
     if (refined)
     {
-        int rc0 = plan->contrib.reserve((size_t)chunk * (size_t)L.nseg * (size_t)width * sizeof(double));
+        int rc0 = plan->contrib.reserve((size_t)chunk * (size_t)L.nseg * (size_t)width * sizeof(double), plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->refineSegs.reserve(sizeof(unsigned long long) * (size_t)L.nseg);
+            rc0 = plan->refineSegs.reserve(sizeof(unsigned long long) * (size_t)L.nseg, plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->refinedTotal.reserve(sizeof(unsigned long long));
+            rc0 = plan->refinedTotal.reserve(sizeof(unsigned long long), plan->owner);
         if (rc0 != CCOIL_OK)
             return rc0;
         cudaError_t e = cudaMemsetAsync(plan->refinedTotal.ptr, 0, sizeof(unsigned long long), st);
@@ -428,13 +359,13 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
     if (ordered)
     {
         const size_t scratch = pointOrderScratchBytes(point_count);
-        int rc0 = plan->orderScratch.reserve(scratch);
+        int rc0 = plan->orderScratch.reserve(scratch, plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->order.reserve(sizeof(int) * (size_t)point_count);
+            rc0 = plan->order.reserve(sizeof(int) * (size_t)point_count, plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->sortedPoints.reserve(inBytes);
+            rc0 = plan->sortedPoints.reserve(inBytes, plan->owner);
         if (rc0 == CCOIL_OK)
-            rc0 = plan->sortedOut.reserve(outBytes);
+            rc0 = plan->sortedOut.reserve(outBytes, plan->owner);
         if (rc0 == CCOIL_OK)
             rc0 = orderPoints(dPoints, point_count, plan->orderScratch.ptr, plan->orderScratch.bytes,
                               static_cast<int *>(plan->order.ptr), static_cast<double *>(plan->sortedPoints.ptr),
@@ -481,27 +412,144 @@ int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, lon
     if (rc == CCOIL_OK && ordered)
         rc = scatterResults(static_cast<const double *>(plan->sortedOut.ptr), static_cast<const int *>(plan->order.ptr),
                             point_count, width, dOut, stream);
-    if (rc != CCOIL_OK)
-        return rc;
+    return rc;
+}
+} // namespace
 
-    if (memory == CCOIL_MEMORY_HOST)
+extern "C" {
+
+int ccoil_abi_version(void) { return CCOIL_ABI_VERSION; }
+
+const char *ccoil_last_error_message(void) { return t_error; }
+
+int ccoil_coil_init(double inner_radius, double thickness, double length, int num_turns, double current,
+                    double sine_frequency, const double position[3], double y_axis_angle, double z_axis_angle,
+                    double precision_factor, int gpu_increments, ccoil_coil_t *out)
+{
+    if (!out)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "out is null");
+    if (!(inner_radius > 0.0) || thickness < 0.0 || length < 0.0 || num_turns < 1 || gpu_increments < 0 ||
+        gpu_increments > kMaxOrder)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT,
+                    "coil needs inner_radius > 0, thickness >= 0, length >= 0, num_turns >= 1, "
+                    "gpu_increments in [0, 100]");
+    initCoil(inner_radius, thickness, length, num_turns, current, sine_frequency, position, y_axis_angle,
+             z_axis_angle, *out);
+    out->precision = coilPrecision(*out, precision_factor, gpu_increments);
+    return CCOIL_OK;
+}
+
+int ccoil_coils_from_params(const double *params, const ccoil_precision_args_t *precisions, int coil_count,
+                            ccoil_coil_t *coils)
+{
+    if (coil_count < 0 || (coil_count > 0 && (!params || !precisions || !coils)))
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "null params, precisions or coils, or coil_count < 0");
+    for (int c = 0; c < coil_count; ++c)
     {
-        cudaError_t e = cudaMemcpyAsync(out, dOut, outBytes, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess)
-            e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess)
-            return cudaFail(e, "field evaluation");
-        long long timeouts = 0;
-        rc = readTimeouts(timeouts);
+        const double *q = params + 9 * c;
+        const int rc = ccoil_coil_init(q[0], q[1], q[2], 1, q[3], 0.0, q + 4, q[7], q[8], 5.0, 0, coils + c);
         if (rc != CCOIL_OK)
             return rc;
-        if (timeouts > g_timeoutsReported.load())
-        {
-            g_timeoutsReported.store(timeouts);
-            return fail(CCOIL_ERR_TIMEOUT, "a staging wait in the field kernel timed out");
-        }
+        coils[c].precision = precisions[c];
     }
     return CCOIL_OK;
+}
+
+int ccoil_precision_arguments(const ccoil_coil_t *coil, double precision_factor, int gpu_increments,
+                              ccoil_precision_args_t *out)
+{
+    if (!coil || !out)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "null argument");
+    if (gpu_increments < 0 || gpu_increments > kMaxOrder)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "gpu_increments must be in [0, 100]");
+    *out = coilPrecision(*coil, precision_factor, gpu_increments);
+    return CCOIL_OK;
+}
+
+int ccoil_pair_arguments(const ccoil_coil_t *primary, const ccoil_coil_t *secondary, double precision_factor,
+                         int gpu_increments, int z_axis_case, int pure_gpu, ccoil_precision_args_t *primary_out,
+                         ccoil_precision_args_t *secondary_out)
+{
+    if (!primary || !secondary || !primary_out || !secondary_out)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "null argument");
+    if (gpu_increments < 0 || gpu_increments > kMaxOrder)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "gpu_increments must be in [0, 100]");
+    pairPrecision(*primary, *secondary, precision_factor, gpu_increments, z_axis_case != 0, pure_gpu != 0,
+                  *primary_out, *secondary_out);
+    return CCOIL_OK;
+}
+
+int ccoil_legendre(int order, double *nodes, double *weights)
+{
+    if (order < 1 || order > kMaxOrder || !nodes || !weights)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "order must be in [1, 100] and buffers non-null");
+    std::memcpy(nodes, legendreNodes(order), sizeof(double) * order);
+    std::memcpy(weights, legendreWeights(order), sizeof(double) * order);
+    return CCOIL_OK;
+}
+
+int ccoil_field_plan_create(const ccoil_coil_t *coils, int coil_count, int field, int precision,
+                            ccoil_field_plan_t **plan)
+{
+    if (!plan)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "plan is null");
+    *plan = nullptr;
+    ccoil_field_plan *p = new (std::nothrow) ccoil_field_plan();
+    if (!p)
+        return fail(CCOIL_ERR_OUT_OF_MEMORY, "host allocation failed");
+    int rc = buildTables(*p, coils, coil_count, field, precision);
+    if (rc == CCOIL_OK && !p->set.blob.empty())
+    {
+        rc = p->tables.reserve(p->set.blob.size(), p->owner);
+        if (rc == CCOIL_OK)
+        {
+            const cudaError_t e =
+                cudaMemcpy(p->tables.ptr, p->set.blob.data(), p->set.blob.size(), cudaMemcpyHostToDevice);
+            if (e != cudaSuccess)
+                rc = cudaFail(e, "cudaMemcpy");
+        }
+    }
+    if (rc != CCOIL_OK)
+    {
+        ccoil_field_plan_destroy(p);
+        return rc;
+    }
+    *plan = p;
+    return CCOIL_OK;
+}
+
+int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, long long point_count, double *out,
+                             int memory, int lanes_per_point, void *stream)
+{
+    if (!plan)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "plan is null");
+    int rc = checkExecute(points, point_count, out, memory);
+    if (rc != CCOIL_OK)
+        return rc;
+    if (lanes_per_point != 0 && !validLanes(lanes_per_point))
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "lanes_per_point must be 0, 1, 2, 4, 8, 16 or 32");
+    if (point_count == 0)
+        return CCOIL_OK;
+    // grid.x limit: 2^31-1 CTAs of 128/lanes points
+    if (point_count > (1LL << 36))
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "point_count above 2^36");
+    if (memory == CCOIL_MEMORY_DEVICE)
+        return runFields(plan, points, point_count, out, lanes_per_point, stream);
+
+    const size_t inBytes = sizeof(double) * 3 * (size_t)point_count;
+    const size_t outBytes = sizeof(double) * (plan->field == CCOIL_FIELD_G ? 9 : 3) * (size_t)point_count;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    rc = plan->points.reserve(inBytes, plan->owner);
+    if (rc == CCOIL_OK)
+        rc = plan->out.reserve(outBytes, plan->owner);
+    if (rc != CCOIL_OK)
+        return rc;
+    cudaError_t e = cudaMemcpyAsync(plan->points.ptr, points, inBytes, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess)
+        return cudaFail(e, "host->device copy of points");
+    rc = runFields(plan, static_cast<const double *>(plan->points.ptr), point_count,
+                   static_cast<double *>(plan->out.ptr), lanes_per_point, stream);
+    return rc == CCOIL_OK ? finishHost(out, static_cast<const double *>(plan->out.ptr), outBytes, st) : rc;
 }
 
 int ccoil_field_plan_segment_count(const ccoil_field_plan_t *plan, int *count)
@@ -516,19 +564,13 @@ int ccoil_field_plan_destroy(ccoil_field_plan_t *plan)
 {
     if (!plan)
         return CCOIL_OK;
-    plan->blob.release();
-    plan->segs.release();
-    plan->points.release();
-    plan->out.release();
-    plan->work.release();
-    plan->workCount.release();
-    plan->contrib.release();
-    plan->refineSegs.release();
-    plan->refinedTotal.release();
-    plan->orderScratch.release();
-    plan->order.release();
-    plan->sortedPoints.release();
-    plan->sortedOut.release();
+    // no kernel on any stream may still use the buffers
+    if (!plan->owner.scoped)
+        cudaDeviceSynchronize();
+    for (DeviceBuffer *b : {&plan->tables, &plan->points, &plan->out, &plan->work, &plan->workCount, &plan->contrib,
+                            &plan->refineSegs, &plan->refinedTotal, &plan->orderScratch, &plan->order,
+                            &plan->sortedPoints, &plan->sortedOut})
+        b->release(plan->owner);
     delete plan;
     return CCOIL_OK;
 }
@@ -537,23 +579,54 @@ int ccoil_compute_fields(const ccoil_coil_t *coils, int coil_count, const double
                          int field, int precision, double *out, int memory, void *stream)
 {
     // the execute step's own checks, before any device work
-    if (point_count < 0 || (point_count > 0 && (!points || !out)))
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "point_count < 0 or null points/out");
-    if (memory != CCOIL_MEMORY_HOST && memory != CCOIL_MEMORY_DEVICE)
-        return fail(CCOIL_ERR_INVALID_ARGUMENT, "memory must be HOST or DEVICE");
-    ccoil_field_plan_t *plan = nullptr;
-    int rc = ccoil_field_plan_create(coils, coil_count, field, precision, &plan);
+    int rc = checkExecute(points, point_count, out, memory);
     if (rc != CCOIL_OK)
         return rc;
-    rc = ccoil_field_plan_execute(plan, points, point_count, out, memory, 0, stream);
-    if (memory == CCOIL_MEMORY_DEVICE && rc == CCOIL_OK)
+    if (point_count > (1LL << 36))
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "point_count above 2^36");
+    ccoil_field_plan *p = new (std::nothrow) ccoil_field_plan();
+    if (!p)
+        return fail(CCOIL_ERR_OUT_OF_MEMORY, "host allocation failed");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    p->owner.scoped = true;
+    p->owner.stream = st;
+    rc = buildTables(*p, coils, coil_count, field, precision);
+    if (rc == CCOIL_OK && point_count > 0)
     {
-        // the plan's device tables must outlive the asynchronous kernel
-        cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-        if (e != cudaSuccess)
-            rc = cudaFail(e, "field evaluation");
+        // one block of device memory for the call: tables, and with host arrays the
+        // points and the results; few points travel with the tables in one copy
+        const size_t inBytes = sizeof(double) * 3 * (size_t)point_count;
+        const size_t outBytes = sizeof(double) * (field == CCOIL_FIELD_G ? 9 : 3) * (size_t)point_count;
+        const bool host = memory == CCOIL_MEMORY_HOST, together = host && inBytes <= kPackedCopyBytes;
+        std::vector<unsigned char> &image = p->set.blob;
+        const size_t pointsAt = (image.size() + 255) / 256 * 256, outAt = (pointsAt + inBytes + 255) / 256 * 256;
+        const size_t tableBytes = image.size();
+        rc = p->tables.reserve(host ? outAt + outBytes : std::max<size_t>(tableBytes, 16), p->owner);
+        if (rc == CCOIL_OK)
+        {
+            unsigned char *base = static_cast<unsigned char *>(p->tables.ptr);
+            if (together)
+            {
+                image.resize(pointsAt + inBytes);
+                std::memcpy(image.data() + pointsAt, points, inBytes);
+            }
+            cudaError_t e = image.empty() ? cudaSuccess
+                                          : cudaMemcpyAsync(base, image.data(), image.size(), cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess && host && !together)
+                e = cudaMemcpyAsync(base + pointsAt, points, inBytes, cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess)
+                rc = cudaFail(e, "host->device copy");
+            double *dOut = host ? reinterpret_cast<double *>(base + outAt) : out;
+            if (rc == CCOIL_OK)
+                rc = runFields(p, host ? reinterpret_cast<const double *>(base + pointsAt) : points, point_count, dOut,
+                               0, stream);
+            if (rc == CCOIL_OK && host)
+                rc = finishHost(out, dOut, outBytes, st);
+            else if (rc == CCOIL_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess)
+                rc = cudaFail(e, "field evaluation");
+        }
     }
-    ccoil_field_plan_destroy(plan);
+    ccoil_field_plan_destroy(p);
     return rc;
 }
 

@@ -508,29 +508,28 @@ extern "C" int ccoil_b_field_adjoint(const double *params, const ccoil_precision
     const long long blocks = point_count > 0 ? (point_count + kAdjPoints - 1) / kAdjPoints : 1;
     if (blocks > (1LL << 24))
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "point_count too large for the adjoint's partial sums");
-    DBuf dBlob, dOff, dPartial;
-    cudaError_t e = dBlob.alloc(blob.size(), st);
+    // one block of device memory: the tables and their offsets, in one copy, and the
+    // partial sums
+    const size_t offAt = (blob.size() + 15) / 16 * 16, partialAt = (offAt + sizeof(long long) * offsets.size() + 255) / 256 * 256;
+    blob.resize(offAt);
+    putBytes(blob, offsets.data(), sizeof(long long) * offsets.size());
+    DBuf arena;
+    cudaError_t e = arena.alloc(partialAt + sizeof(double) * 9 * coil_count * blocks, st);
     if (e == cudaSuccess)
-        e = dOff.alloc(sizeof(long long) * offsets.size(), st);
-    if (e == cudaSuccess)
-        e = dPartial.alloc(sizeof(double) * 9 * coil_count * blocks, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dBlob.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dOff.p, offsets.data(), sizeof(long long) * offsets.size(), cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(arena.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess)
         return cudaFail(e, "adjoint set-up");
+    const unsigned char *base = static_cast<const unsigned char *>(arena.p);
+    double *partial = reinterpret_cast<double *>(static_cast<unsigned char *>(arena.p) + partialAt);
     if (point_count == 0)
-        e = cudaMemsetAsync(dPartial.p, 0, sizeof(double) * 9 * coil_count, st);
+        e = cudaMemsetAsync(partial, 0, sizeof(double) * 9 * coil_count, st);
     else
         adjointKernel<<<dim3((unsigned)blocks, (unsigned)std::min(coil_count, 65535)), kAdjThreads, 0, st>>>(
-            static_cast<const unsigned char *>(dBlob.p), static_cast<const long long *>(dOff.p), coil_count, points,
-            grad_b, point_count, static_cast<double *>(dPartial.p));
+            base, reinterpret_cast<const long long *>(base + offAt), coil_count, points, grad_b, point_count, partial);
     if (e == cudaSuccess)
         e = cudaGetLastError();
     if (e == cudaSuccess)
-        adjointReduce<<<(coil_count * 9 + 31) / 32, 1024, 0, st>>>(static_cast<const double *>(dPartial.p),
-                                                                    (int)blocks, coil_count, grad_params);
+        adjointReduce<<<(coil_count * 9 + 31) / 32, 1024, 0, st>>>(partial, (int)blocks, coil_count, grad_params);
     if (e == cudaSuccess)
         e = cudaGetLastError();
     if (e == cudaSuccess)

@@ -209,6 +209,9 @@ double refineFraction();  // the process-wide fraction (ccoil_set_refine_fractio
 constexpr size_t kRefineContribBytes = size_t(1) << 32;
 constexpr unsigned long long kRefineListPairs = 1ULL << 28;
 int launchFields(const FieldLaunch &L, void *stream);
+// whether this build's field kernels have bounded waits whose timeouts a call reports
+// (only the staged variants have)
+bool fieldKernelsWait();
 // CTAs of 128 threads that one SM holds of the kernel for (field, precision)
 int fieldBlocksPerSM(int field, int precision);
 int readTimeouts(long long &count);
@@ -255,9 +258,17 @@ struct PairOptions
     bool full_ring = false;
     double scale = 1.0;
 };
+// poses of the arrangements: packed ccoil_pose_t rows (host or device memory), or
+// separate host arrays
+struct PoseSource
+{
+    const double *packed = nullptr;
+    const double *position = nullptr, *yAngle = nullptr, *zAngle = nullptr;
+    bool given() const { return packed || position; }
+};
 int pairArrangements(const ccoil_coil_t *primaries, int primary_count, const ccoil_coil_t *secondary,
                      const ccoil_precision_args_t *secondary_precisions, const ccoil_precision_args_t *zaxis_precisions,
-                     const ccoil_pose_t *primary_poses, const ccoil_pose_t *secondary_poses, long long count,
+                     const PoseSource &primary_poses, const PoseSource &secondary_poses, long long count,
                      int quantity, int precision, double *out, long long *z_axis_count, int memory, void *stream,
                      const PairOptions &opt);
 int launchBatch(const BatchLaunch &B, void *stream);

@@ -385,6 +385,8 @@ int launchFields(const FieldLaunch &L, void *stream)
     return CCOIL_OK;
 }
 
+bool fieldKernelsWait() { return CCOIL_FP32_STAGE || CCOIL_FP64_STAGE; }
+
 int fieldBlocksPerSM(int field, int precision)
 {
     if (precision == CCOIL_PRECISION_FP64)

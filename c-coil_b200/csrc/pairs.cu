@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -1330,6 +1331,25 @@ struct DevBuf
             cudaFreeAsync(p, st);
     }
 };
+
+// poses and results up to this size share a copy with a call's tables and counters
+constexpr size_t kPackedBytes = size_t(1) << 16;
+
+void packHostPoses(const PoseSource &s, long long n, double *dst)
+{
+    if (s.packed)
+    {
+        std::memcpy(dst, s.packed, sizeof(ccoil_pose_t) * (size_t)n);
+        return;
+    }
+    for (long long i = 0; i < n; ++i)
+    {
+        for (int k = 0; k < 3; ++k)
+            dst[5 * i + k] = s.position[3 * i + k];
+        dst[5 * i + 3] = s.yAngle[i];
+        dst[5 * i + 4] = s.zAngle[i];
+    }
+}
 } // namespace
 
 int cudaFail(cudaError_t e, const char *what);
@@ -1339,20 +1359,21 @@ using namespace ccoil;
 
 int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, const ccoil_coil_t *secondary,
                             const ccoil_precision_args_t *secondary_precisions,
-                            const ccoil_precision_args_t *zaxis_precisions, const ccoil_pose_t *primary_poses,
-                            const ccoil_pose_t *secondary_poses, long long count, int quantity, int precision,
-                            double *out, long long *z_axis_count, int memory, void *stream, const PairOptions &opt)
+                            const ccoil_precision_args_t *zaxis_precisions, const PoseSource &prim,
+                            const PoseSource &sec, long long count, int quantity, int precision, double *out,
+                            long long *z_axis_count, int memory, void *stream, const PairOptions &opt)
 {
+    const bool havePrim = prim.given(), split_poses = sec.position != nullptr || prim.position != nullptr;
     if (primary_count < 0 || (primary_count > 0 && (!primaries || !secondary_precisions)) || !secondary)
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "null coils or negative primary_count");
-    if (count < 0 || (count > 0 && (!secondary_poses || !out)))
+    if (count < 0 || (count > 0 && (!sec.given() || !out)))
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "count < 0 or null poses/out");
-    if (primary_poses && primary_count != 1)
+    if (havePrim && primary_count != 1)
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "per-arrangement primary poses need exactly one primary");
     if (quantity != CCOIL_PAIR_MUTUAL_INDUCTANCE && quantity != CCOIL_PAIR_FORCE_TORQUE &&
         quantity != CCOIL_PAIR_MUTUAL_INDUCTANCE_GRADIENT && quantity != CCOIL_PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT)
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "unknown pair quantity");
-    if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT && count > 0 && (primary_count != 1 || !primary_poses))
+    if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE_PARAMETER_GRADIENT && count > 0 && (primary_count != 1 || !havePrim))
         return failMessage(CCOIL_ERR_INVALID_ARGUMENT,
                            "the parameter gradient needs exactly one primary with per-arrangement poses");
     if (precision != CCOIL_PRECISION_FP64 && precision != CCOIL_PRECISION_FP32_COMPENSATED &&
@@ -1407,59 +1428,26 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
             if (!buildZAxis(primaries[j], *secondary, zaxis_precisions[2 * j], zaxis_precisions[2 * j + 1], blob, err))
                 return fail(CCOIL_ERR_INVALID_ARGUMENT, "primary " + std::to_string(j) + ": " + err);
         }
-    DevBuf dBlob, dOff, dPrim, dSec, dOut, dZ, dZOff, dZList, dZCount, dScratch, dPartial;
-    cudaError_t e = dBlob.alloc(blob.size(), st);
-    if (e == cudaSuccess)
-        e = dOff.alloc(sizeof(long long) * offsets.size(), st);
-    if (e == cudaSuccess)
-        e = dZ.alloc(sizeof(unsigned long long), st);
-    if (e == cudaSuccess && zPass)
-    {
-        e = dZOff.alloc(sizeof(long long) * primary_count, st);
-        if (e == cudaSuccess)
-            e = dZList.alloc(sizeof(long long) * count, st);
-        if (e == cudaSuccess)
-            e = dZCount.alloc(sizeof(unsigned long long), st);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(dZOff.p, zOffsets.data(), sizeof(long long) * primary_count, cudaMemcpyHostToDevice,
-                                st);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(dZCount.p, 0, sizeof(unsigned long long), st);
-    }
-    if (e == cudaSuccess && memory == CCOIL_MEMORY_HOST)
-    {
-        e = dSec.alloc(sizeof(double) * 5 * count, st);
-        if (e == cudaSuccess && primary_poses)
-            e = dPrim.alloc(sizeof(double) * 5 * count, st);
-        if (e == cudaSuccess)
-            e = dOut.alloc(sizeof(double) * width * count, st);
-    }
-    if (e != cudaSuccess)
-        return cudaFail(e, "scratch allocation");
-    e = cudaMemcpyAsync(dBlob.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dOff.p, offsets.data(), sizeof(long long) * offsets.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(dZ.p, 0, sizeof(unsigned long long), st);
-    const double *secP = reinterpret_cast<const double *>(secondary_poses);
-    const double *primP = reinterpret_cast<const double *>(primary_poses);
-    double *o = out;
-    if (e == cudaSuccess && memory == CCOIL_MEMORY_HOST)
-    {
-        e = cudaMemcpyAsync(dSec.p, secondary_poses, sizeof(double) * 5 * count, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess && primary_poses)
-            e = cudaMemcpyAsync(dPrim.p, primary_poses, sizeof(double) * 5 * count, cudaMemcpyHostToDevice, st);
-        secP = static_cast<const double *>(dSec.p);
-        primP = primary_poses ? static_cast<const double *>(dPrim.p) : nullptr;
-        o = static_cast<double *>(dOut.p);
-    }
-    if (e != cudaSuccess)
-        return cudaFail(e, "host->device copy");
-    // one primary whose tables fit: stage them in shared memory
-    const int stagedBytes = (primary_count == 1 && generalBytes <= CCOIL_PAIR_STAGE_MAX_BYTES &&
-                             generalBytes % 16 == 0)
-                                ? (int)generalBytes
-                                : 0;
+    // One block of device memory for the call.  First what is uploaded, in one copy:
+    // tables, offsets, the two z-axis counters (zero) and the poses, unless they are a
+    // large array that can be copied as it is; after them the results, so that few results come back in one copy with
+    // the counters; then what stays on the device.
+    const bool host = memory == CCOIL_MEMORY_HOST;
+    const size_t poseBytes = sizeof(ccoil_pose_t) * (size_t)count, outBytes = sizeof(double) * width * (size_t)count;
+    const bool packPoses = host && (split_poses || poseBytes <= kPackedBytes), packOut = host && outBytes <= kPackedBytes;
+    size_t arenaBytes = 0;
+    auto region = [&](size_t bytes) {
+        const size_t at = arenaBytes;
+        arenaBytes += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t atBlob = region(blob.size()), atOff = region(sizeof(long long) * offsets.size()),
+                 atZOff = region(sizeof(long long) * zOffsets.size());
+    const size_t atSec = packPoses ? region(poseBytes) : 0, atPrim = packPoses && havePrim ? region(poseBytes) : 0;
+    const size_t atCount = region(2 * sizeof(unsigned long long)), uploadBytes = arenaBytes;
+    const size_t atOut = region(host ? outBytes : 0), atZList = region(zPass ? sizeof(long long) * count : 0);
+    const size_t atBigSec = region(host && !packPoses ? poseBytes : 0);
+    const size_t atBigPrim = region(host && !packPoses && havePrim ? poseBytes : 0);
     int secNodes = 0;
     for (long long off : offsets)
     {
@@ -1487,18 +1475,14 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     // 9.9: each warp's last FP64 batch of 32 nodes is partly empty)
     const int team = !refine ? 1 : count <= 148LL * 3 ? 12 : count <= resident * 3 ? 4 : 1;
     const long long perArr = (long long)split.groups * split.parts;
-    if (perArr > 1)
-    {
-        e = dPartial.alloc(sizeof(double) * (size_t)width * (size_t)(count * perArr), st);
-        if (e != cudaSuccess)
-            return cudaFail(e, "arrangement partial sums");
-    }
+    const size_t atPartial = region(perArr > 1 ? sizeof(double) * (size_t)width * (size_t)(count * perArr) : 0);
     long long blocks = team > 1 ? count : (count * perArr + 3) / 4;
     if (blocks > 148LL * 64)
         blocks = 148LL * 64;
     // FP32_REFINED: every warp's region of node contributions (the grid strides over
     // the arrangements, so the scratch is sized by the grid, not by the count)
     const int scratchNodes = refine ? secNodes : 0;
+    size_t scratchBytes = 0;
     if (refine)
     {
         // at most kPairRefineScratchBytes: a secondary with many nodes runs on fewer
@@ -1506,20 +1490,56 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         const size_t perBlock = sizeof(double) * (size_t)width * (size_t)scratchNodes * (team > 1 ? 1 : 4);
         const long long fit = (long long)(kPairRefineScratchBytes / perBlock);
         blocks = std::max(1LL, std::min(blocks, std::max(fit, 148LL)));
-        e = dScratch.alloc(perBlock * (size_t)blocks, st);
-        if (e != cudaSuccess)
-            return cudaFail(e, "refinement scratch");
+        scratchBytes = perBlock * (size_t)blocks;
     }
+    const size_t atScratch = region(scratchBytes);
+    DevBuf arena;
+    cudaError_t e = arena.alloc(arenaBytes, st);
+    if (e != cudaSuccess)
+        return cudaFail(e, "device memory of the call");
+    unsigned char *base = static_cast<unsigned char *>(arena.p);
+    const size_t backBytes = packOut ? atOut - atCount + outBytes : 0;  // counters and results
+    std::unique_ptr<unsigned char[]> image(new (std::nothrow) unsigned char[std::max(uploadBytes, backBytes)]);
+    if (!image)
+        return failMessage(CCOIL_ERR_OUT_OF_MEMORY, "host allocation failed");
+    std::memcpy(image.get() + atBlob, blob.data(), blob.size());
+    std::memcpy(image.get() + atOff, offsets.data(), sizeof(long long) * offsets.size());
+    std::memcpy(image.get() + atZOff, zOffsets.data(), sizeof(long long) * zOffsets.size());
+    std::memset(image.get() + atCount, 0, 2 * sizeof(unsigned long long));
+    if (packPoses)
+    {
+        packHostPoses(sec, count, reinterpret_cast<double *>(image.get() + atSec));
+        if (havePrim)
+            packHostPoses(prim, count, reinterpret_cast<double *>(image.get() + atPrim));
+    }
+    e = cudaMemcpyAsync(base, image.get(), uploadBytes, cudaMemcpyHostToDevice, st);
+    const double *secP = sec.packed, *primP = prim.packed;
+    if (host)
+    {
+        secP = reinterpret_cast<const double *>(base + (packPoses ? atSec : atBigSec));
+        primP = havePrim ? reinterpret_cast<const double *>(base + (packPoses ? atPrim : atBigPrim)) : nullptr;
+        if (e == cudaSuccess && !packPoses)
+            e = cudaMemcpyAsync(base + atBigSec, sec.packed, poseBytes, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && !packPoses && havePrim)
+            e = cudaMemcpyAsync(base + atBigPrim, prim.packed, poseBytes, cudaMemcpyHostToDevice, st);
+    }
+    if (e != cudaSuccess)
+        return cudaFail(e, "host->device copy");
+    double *o = host ? reinterpret_cast<double *>(base + atOut) : out;
+    // one primary whose tables fit: stage them in shared memory
+    const int stagedBytes = (primary_count == 1 && generalBytes <= CCOIL_PAIR_STAGE_MAX_BYTES &&
+                             generalBytes % 16 == 0)
+                                ? (int)generalBytes
+                                : 0;
     const double fraction = refineFraction();
-    auto *scratch = static_cast<double *>(dScratch.p);
-    auto *partial = static_cast<double *>(dPartial.p);
-    auto *zc = static_cast<unsigned long long *>(dZ.p);
-    const auto *dB = static_cast<const unsigned char *>(dBlob.p);
-    const auto *dO = static_cast<const long long *>(dOff.p);
+    auto *scratch = reinterpret_cast<double *>(base + atScratch);
+    auto *partial = perArr > 1 ? reinterpret_cast<double *>(base + atPartial) : nullptr;
+    auto *zc = reinterpret_cast<unsigned long long *>(base + atCount), *zN = zc + 1;
+    const unsigned char *dB = base + atBlob;
+    const auto *dO = reinterpret_cast<const long long *>(base + atOff);
     const size_t smem = (size_t)stagedBytes;
-    const auto *zO = static_cast<const long long *>(dZOff.p);
-    auto *zL = static_cast<long long *>(dZList.p);
-    auto *zN = static_cast<unsigned long long *>(dZCount.p);
+    const auto *zO = zPass ? reinterpret_cast<const long long *>(base + atZOff) : nullptr;
+    auto *zL = reinterpret_cast<long long *>(base + atZList);
 #define CCOIL_PAIR_LAUNCH(Q, F, ...)                                                                                   \
     pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, pairThreads(team), smem, st>>>(                                          \
         dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction,  \
@@ -1584,16 +1604,28 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return cudaFail(e, "pair kernel launch");
-    if (memory == CCOIL_MEMORY_HOST)
-        e = cudaMemcpyAsync(out, o, sizeof(double) * width * count, cudaMemcpyDeviceToHost, st);
-    unsigned long long zcount = 0;
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&zcount, zc, sizeof(zcount), cudaMemcpyDeviceToHost, st);
     // the call is synchronous, as the reference's: host outputs and the z-axis count
+    unsigned long long zcount = 0;
+    if (packOut)
+    {
+        e = cudaMemcpyAsync(image.get(), base + atCount, backBytes, cudaMemcpyDeviceToHost, st);
+    }
+    else
+    {
+        if (host)
+            e = cudaMemcpyAsync(out, o, outBytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&zcount, zc, sizeof(zcount), cudaMemcpyDeviceToHost, st);
+    }
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
     if (e != cudaSuccess)
         return cudaFail(e, "pair arrangements");
+    if (packOut)
+    {
+        std::memcpy(&zcount, image.get(), sizeof(zcount));
+        std::memcpy(out, image.get() + (atOut - atCount), outBytes);
+    }
     if (z_axis_count)
         *z_axis_count = (long long)zcount;
     return CCOIL_OK;
@@ -1607,9 +1639,37 @@ extern "C" int ccoil_pair_arrangements_zaxis(const ccoil_coil_t *primaries, int 
                                              long long count, int quantity, int precision, double *out,
                                              long long *z_axis_count, int memory, void *stream)
 {
-    return pairArrangements(primaries, primary_count, secondary, secondary_precisions, zaxis_precisions,
-                            primary_poses, secondary_poses, count, quantity, precision, out, z_axis_count, memory,
-                            stream, PairOptions{});
+    PoseSource prim, sec;
+    prim.packed = reinterpret_cast<const double *>(primary_poses);
+    sec.packed = reinterpret_cast<const double *>(secondary_poses);
+    return pairArrangements(primaries, primary_count, secondary, secondary_precisions, zaxis_precisions, prim, sec,
+                            count, quantity, precision, out, z_axis_count, memory, stream, PairOptions{});
+}
+
+extern "C" int ccoil_pair_arrangements_arrays(const ccoil_coil_t *primaries, int primary_count,
+                                              const ccoil_coil_t *secondary,
+                                              const ccoil_precision_args_t *secondary_precisions,
+                                              const ccoil_precision_args_t *zaxis_precisions,
+                                              const ccoil_pose_arrays_t *primary_poses,
+                                              const ccoil_pose_arrays_t *secondary_poses, long long count,
+                                              int quantity, int precision, double *out, long long *z_axis_count,
+                                              void *stream)
+{
+    auto source = [](const ccoil_pose_arrays_t *a) {
+        PoseSource s;
+        if (a && a->position && a->y_angle && a->z_angle)
+        {
+            s.position = a->position;
+            s.yAngle = a->y_angle;
+            s.zAngle = a->z_angle;
+        }
+        return s;
+    };
+    const PoseSource prim = source(primary_poses), sec = source(secondary_poses);
+    if (primary_poses && count > 0 && !prim.given())
+        return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "null primary pose arrays");
+    return pairArrangements(primaries, primary_count, secondary, secondary_precisions, zaxis_precisions, prim, sec,
+                            count, quantity, precision, out, z_axis_count, CCOIL_MEMORY_HOST, stream, PairOptions{});
 }
 
 extern "C" int ccoil_pair_arrangements(const ccoil_coil_t *primaries, int primary_count, const ccoil_coil_t *secondary,

@@ -195,9 +195,11 @@ void pairs(const Coil *prims, int primCount, const Coil &sec, const std::vector<
     PairOptions opt;
     opt.full_ring = true;
     opt.scale = correctionFactor / (2.0 * kPi);
-    check(pairArrangements(prims, primCount, &sec, secPrec.data(), nullptr, primPoses ? primPoses->data() : nullptr,
-                           secPoses.data(), count, quantity, CCOIL_PRECISION_FP64, out, nullptr, CCOIL_MEMORY_HOST,
-                           nullptr, opt),
+    PoseSource primSource, secSource;
+    primSource.packed = primPoses ? reinterpret_cast<const double *>(primPoses->data()) : nullptr;
+    secSource.packed = reinterpret_cast<const double *>(secPoses.data());
+    check(pairArrangements(prims, primCount, &sec, secPrec.data(), nullptr, primSource, secSource, count, quantity,
+                           CCOIL_PRECISION_FP64, out, nullptr, CCOIL_MEMORY_HOST, nullptr, opt),
           where);
 }
 

@@ -294,6 +294,24 @@ int ccoil_pair_arrangements_zaxis(const ccoil_coil_t *primaries, int primary_cou
                                   const ccoil_pose_t *secondary_poses, long long count, int quantity, int precision,
                                   double *out, long long *z_axis_count, int memory, void *stream);
 
+/* Poses as the separate arrays in which the reference's arrangement methods take
+ * them: n x 3 positions and n angles each, host memory. */
+typedef struct ccoil_pose_arrays
+{
+    const double *position;
+    const double *y_angle;
+    const double *z_angle;
+} ccoil_pose_arrays_t;
+
+/* ccoil_pair_arrangements_zaxis with host memory for poses and results, the
+ * poses as separate arrays (primary_poses NULL: the primaries keep their own). */
+int ccoil_pair_arrangements_arrays(const ccoil_coil_t *primaries, int primary_count, const ccoil_coil_t *secondary,
+                                   const ccoil_precision_args_t *secondary_precisions,
+                                   const ccoil_precision_args_t *zaxis_precisions,
+                                   const ccoil_pose_arrays_t *primary_poses,
+                                   const ccoil_pose_arrays_t *secondary_poses, long long count, int quantity,
+                                   int precision, double *out, long long *z_axis_count, void *stream);
+
 /* Self inductance of `count` coils (Coil::computeAndSetSelfInductance,
  * src/Coil/MInductance/ComputeMInductanceMethods.cxx:55-81):
  * pair_precisions[2c] and [2c+1] are the coil's pair arguments with itself in
@@ -338,6 +356,11 @@ int ccoil_batch_plan_destroy(ccoil_batch_plan_t *plan);
 /* ------------------------------------------------------------------------ *
  * Adjoint                                                                   *
  * ------------------------------------------------------------------------ */
+
+/* Coils from parameter rows {R, a, b, N*I, x, y, z, y_axis_angle, z_axis_angle}
+ * (one turn, current N*I), each at the given PrecisionArguments. */
+int ccoil_coils_from_params(const double *params, const ccoil_precision_args_t *precisions, int coil_count,
+                            ccoil_coil_t *coils);
 
 /* Gradient of a loss L(B) with respect to each coil's parameters, given
  * grad_b = dL/dB at the points (no counterpart in the reference, which has no
