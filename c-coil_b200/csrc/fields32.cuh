@@ -263,8 +263,10 @@ __device__ __forceinline__ bool isNearPair(const unsigned char *blob, const Segm
     return nearWinding(h, toCoilFrame(h, px, py, pz));
 }
 
-// Lists the near-field pairs, one thread per point: the pairs of a point in one
-// run of entries, in segment order.  It takes every frame transform once more.
+// Lists the near-field pairs: the pairs of a point in one run of entries, in segment
+// order.  It takes every frame transform once more.  LANES (1 or 32) threads per
+// point share its segments.
+template <int LANES>
 __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__restrict__ blob,
                                                          const SegmentDesc *__restrict__ segs, int nseg,
                                                          const double *__restrict__ points, long long npts,
@@ -272,28 +274,41 @@ __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__
                                                          unsigned long long workCapacity,
                                                          unsigned long long *__restrict__ workCount)
 {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x % LANES;
+    const long long p = (long long)blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
     if (p >= npts)
         return;
     const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
     int count = 0, first = nseg;
 #pragma unroll 2
-    for (int s = 0; s < nseg; ++s)
+    for (int s = lane; s < nseg; s += LANES)
         if (isNearPair(blob, segs, s, px, py, pz))
         {
-            first = count == 0 ? s : first;
+            first = min(first, s);
             ++count;
         }
+    if (LANES > 1)
+    {
+        count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
+        first = (int)__reduce_min_sync(0xffffffffu, (unsigned)first);
+    }
     if (count == 0)
         return;
-    unsigned long long slot = atomicAdd(workCount, (unsigned long long)count);
-    for (int s = first; s < nseg && slot < workCapacity; ++s)
-        if (isNearPair(blob, segs, s, px, py, pz))
+    unsigned long long slot = lane == 0 ? atomicAdd(workCount, (unsigned long long)count) : 0ull;
+    if (LANES > 1)
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+    for (int s0 = first / LANES * LANES; s0 < nseg && slot < workCapacity; s0 += LANES)
+    {
+        const bool near = s0 + lane < nseg && isNearPair(blob, segs, s0 + lane, px, py, pz);
+        const unsigned before = LANES > 1 ? __ballot_sync(0xffffffffu, near) : (near ? 1u : 0u);
+        const unsigned long long at = slot + __popc(before & ((1u << lane) - 1u));
+        if (near && at < workCapacity)
         {
-            work[slot].point = (int)p;
-            work[slot].segment = s;
-            ++slot;
+            work[at].point = (int)p;
+            work[at].segment = s0 + lane;
         }
+        slot += __popc(before);
+    }
 }
 
 // Evaluates the near-field pairs: one warp per point's run of entries, the FP64
@@ -355,14 +370,14 @@ __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__re
 
 // One segment at one point for the refinement pass: the vector potential (and
 // E) and the field with the forms above, the gradient with the FP64 field
-// integrands
-template <int FIELD>
+// integrands; LANES neighbouring lanes split the angular nodes
+template <int FIELD, int LANES>
 __device__ __forceinline__ void integrateSegmentRefine(const unsigned char *seg, double px, double py, double pz,
-                                                       double *acc)
+                                                       int lane, double *acc)
 {
     if (FIELD == CCOIL_FIELD_G)
     {
-        integrateSegment64<FIELD, 1>(seg, px, py, pz, 0, acc);
+        integrateSegment64<FIELD, LANES>(seg, px, py, pz, lane, acc);
         return;
     }
     const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
@@ -373,50 +388,83 @@ __device__ __forceinline__ void integrateSegmentRefine(const unsigned char *seg,
     if (FIELD == CCOIL_FIELD_B)
     {
         double H, Z;
-        segmentB64Fast(h, tt, lt, pt, f, H, Z);
+        segmentB64Fast<LANES>(h, tt, lt, pt, f, lane, H, Z);
         addRotated(h, H * f.cphi, H * f.sphi, Z, acc);
     }
     else
     {
-        const double a = segmentA64Fast<true>(h, tt, lt, pt, f) * h.field_factor;
+        const double a = segmentA64Fast<true, LANES>(h, tt, lt, pt, f, lane) * h.field_factor;
         addRotated(h, -a * f.sphi, a * f.cphi, 0.0, acc);
     }
 }
 
-// FP32_REFINED's FP64 pass: one thread per listed (point, segment) pair, the
-// whole segment in FP64 (integrateSegmentRefine; each thickness node's set-up
-// serves all its angular nodes, as in the FP64 field kernel, where one warp
-// per pair measured 1.2x the time), the result added to the point's output
-// (FP64 atomics).  The selection lists the pairs segment-major, so the lanes
-// of a warp read one segment's tables and run loops of the same length.
-// Grid-stride over the device-side count.
+// FP32_REFINED's FP64 pass: LANES threads per listed (point, segment) pair, the
+// result added to the point's output (FP64 atomics).  One thread per pair while
+// there are enough of them (each thickness node's set-up serves all its angular
+// nodes, as in the FP64 field kernel, where one warp per pair measured 1.2x the
+// time): the selection lists the pairs segment-major, so the lanes of a warp read
+// one segment's tables and run loops of the same length.  With fewer pairs than
+// threads, 4, 16 or 32 of them share a pair.  The kernel picks by the device-side
+// count (this pass for A of 15 coils at 389 points, 1,500 pairs: 263 us with one
+// thread per pair, 59 us with 32).
 // CTAs per SM of the FP64 pair pass: several nodes in flight per thread without
 // spills (vector potential 120 registers, field 112, gradient 142) measured 1 %
 // faster for the whole call than the most CTAs that fit without (6, 5 and 4)
 constexpr int refineMinBlocks(int field) { return field == CCOIL_FIELD_G ? 3 : 4; }
+template <int FIELD, int LANES>
+__device__ __forceinline__ void refinePairs(const unsigned char *__restrict__ blob,
+                                            const SegmentDesc *__restrict__ segs, const double *__restrict__ points,
+                                            double *__restrict__ out, const NearPair *__restrict__ work,
+                                            unsigned long long n)
+{
+    constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
+    const int lane = threadIdx.x % LANES;
+    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x / LANES;
+    const unsigned long long rounds = (n + stride - 1) / stride;  // the same for all lanes of a warp
+    unsigned long long i = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    for (unsigned long long r = 0; LANES == 1 ? i < n : r < rounds; ++r, i += stride)
+    {
+        const bool valid = LANES == 1 || i < n;
+        double acc[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            acc[k] = 0.0;
+        long long p = 0;
+        if (valid)
+        {
+            const NearPair e = work[i];
+            p = e.point;
+            integrateSegmentRefine<FIELD, LANES>(blob + segs[e.segment].offset, points[3 * p], points[3 * p + 1],
+                                                 points[3 * p + 2], lane, acc);
+        }
+#pragma unroll
+        for (int off = LANES / 2; off > 0; off /= 2)
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+        if (valid && lane == 0)
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                atomicAdd(&out[W * p + k], acc[k]);
+    }
+}
+
 template <int FIELD>
 __global__ void __launch_bounds__(128, refineMinBlocks(FIELD)) refinePairsKernel64(
     const unsigned char *__restrict__ blob, const SegmentDesc *__restrict__ segs, const double *__restrict__ points,
     double *__restrict__ out, const NearPair *__restrict__ work, unsigned long long workCapacity,
     const unsigned long long *__restrict__ workCount)
 {
-    constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
     const unsigned long long n = min(*workCount, workCapacity);
-    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    {
-        const NearPair e = work[i];
-        const long long p = e.point;
-        double acc[W];
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            acc[k] = 0.0;
-        integrateSegmentRefine<FIELD>(blob + segs[e.segment].offset, points[3 * p], points[3 * p + 1],
-                                      points[3 * p + 2], acc);
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            atomicAdd(&out[W * p + k], acc[k]);
-    }
+    const unsigned long long threads = (unsigned long long)gridDim.x * blockDim.x;
+    if (n >= threads)
+        refinePairs<FIELD, 1>(blob, segs, points, out, work, n);
+    else if (4 * n >= threads)
+        refinePairs<FIELD, 4>(blob, segs, points, out, work, n);
+    else if (16 * n >= threads)
+        refinePairs<FIELD, 16>(blob, segs, points, out, work, n);
+    else
+        refinePairs<FIELD, 32>(blob, segs, points, out, work, n);
 }
 
 // FP32_REFINED selection.  A pair is picked when its stored contribution's

@@ -11,7 +11,8 @@
 // namespaces after integrands64.cuh; the reciprocal square roots, square roots
 // and divisions come from fp64ops.cuh.
 
-// The vector potential of one segment at one point, one thread.  Fast method:
+// The vector potential of one segment at one point; LANES lanes split the angular
+// nodes (or mirror pairs) and hold partial sums.  Fast method:
 // the reference's node value is log((e1 + d1) / (e2 + d2)) =
 // asinh(top / sqrt(D)) - asinh(bot / sqrt(D)) (D = p^2 + r^2 - 2 p r c,
 // e = sqrt(d^2 + 1)).  With A1 = |top| + s1, A2 = |bot| + s2,
@@ -37,8 +38,8 @@ template <bool CHECKED> __device__ __forceinline__ double logRatio64t(double n, 
 }
 
 // One thickness node of the fast method: sum over the angular nodes.
-template <bool PAIRED, bool CHECKED>
-__device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, double cA, double cB, double T2, double B2,
+template <bool PAIRED, bool CHECKED, int LANES>
+__device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, int lane, double cA, double cB, double T2, double B2,
                                              double aT, double aB, bool above, bool below)
 {
     auto ratio = [&](double c, double &num, double &den) {
@@ -53,7 +54,7 @@ __device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, double cA
     // this within 56 registers
     constexpr int kUnroll = PAIRED ? 2 : 1;
 #pragma unroll kUnroll
-    for (int m = 0; m < n / 2; ++m)
+    for (int m = lane; m < n / 2; m += LANES)
     {
         const double2 q = pt[PAIRED ? 2 * m : m], qm = pt[PAIRED ? 2 * m + 1 : n - 1 - m];
         double n1, e1, n2, e2;
@@ -61,7 +62,7 @@ __device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, double cA
         ratio(qm.x, n2, e2);
         part += 0.5 * (q.y * q.x - qm.y * qm.x) * logRatio64t<CHECKED>(n1 * e2, e1 * n2);
     }
-    if (n & 1)
+    if ((n & 1) && lane == 0)
     {
         // an odd table's middle node
         const double2 q = pt[PAIRED ? n - 1 : n / 2];
@@ -72,9 +73,9 @@ __device__ __forceinline__ double phiLoopA64(const double2 *pt, int n, double cA
     return part;
 }
 
-template <bool PAIRED>
+template <bool PAIRED, int LANES = 1>
 __device__ __forceinline__ double segmentA64Fast(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                                   const double2 *pt, const Frame &f)
+                                                 const double2 *pt, const Frame &f, int lane = 0)
 {
     double sum = 0.0;
     const int n = h.n_phi;
@@ -93,8 +94,9 @@ __device__ __forceinline__ double segmentA64Fast(const SegmentHeader &h, const d
             // FP64's normal range with them
             const double k = fabs(cA);
             const bool fast = inRange64(cB - k, fmax(T2, B2) + (cB + k));
-            const double part = fast ? phiLoopA64<PAIRED, false>(pt, n, cA, cB, T2, B2, aT, aB, above, below)
-                                     : phiLoopA64<PAIRED, true>(pt, n, cA, cB, T2, B2, aT, aB, above, below);
+            const double part =
+                fast ? phiLoopA64<PAIRED, false, LANES>(pt, n, lane, cA, cB, T2, B2, aT, aB, above, below)
+                     : phiLoopA64<PAIRED, true, LANES>(pt, n, lane, cA, cB, T2, B2, aT, aB, above, below);
             sum += t.y * t.x * part;
         }
     }
@@ -110,13 +112,13 @@ __device__ __forceinline__ double segmentA64Fast(const SegmentHeader &h, const d
                 const double cA = 2.0 * t.x * f.r, cB = t.x * t.x + f.r * f.r + zl * zl;
                 double part = 0.0;
                 if (inRange64(cB - fabs(cA), cB + fabs(cA)))
-                    for (int k = 0; k < n; ++k)
+                    for (int k = lane; k < n; k += LANES)
                     {
                         const double2 q = pt[k];
                         part += q.y * q.x * rsqrt64u(cB - cA * q.x);
                     }
                 else
-                    for (int k = 0; k < n; ++k)
+                    for (int k = lane; k < n; k += LANES)
                     {
                         const double2 q = pt[k];
                         part += q.y * q.x * rsqrt64(cB - cA * q.x);
@@ -128,16 +130,16 @@ __device__ __forceinline__ double segmentA64Fast(const SegmentHeader &h, const d
     return sum;
 }
 
-// The field of one segment at one point, one thread, four nodes in flight:
+// The field of one segment at one point, LANES lanes likewise, four nodes in flight:
 // the reference's node values with every 1/sqrt(D) from rsqrt64 (fast method:
 // w c (g2 - g1) and w (p^2 - p r c) / rho^2 (top g1 - bot g2); slow method:
 // w g^3 (p^2 - p r c) and w g^3 p zl c)
-template <bool CHECKED>
-__device__ __forceinline__ void phiLoopB64(const double2 *pt, int n, double cA, double cB, double cC, double d1,
+template <bool CHECKED, int LANES>
+__device__ __forceinline__ void phiLoopB64(const double2 *pt, int n, int lane, double cA, double cB, double cC, double d1,
                                            double d2, double top, double bot, double &h0, double &z0)
 {
 #pragma unroll 4
-    for (int k = 0; k < n; ++k)
+    for (int k = lane; k < n; k += LANES)
     {
         const double2 q = pt[k];
         const double F = 2.0 * cB * q.x;
@@ -147,8 +149,9 @@ __device__ __forceinline__ void phiLoopB64(const double2 *pt, int n, double cA, 
     }
 }
 
+template <int LANES = 1>
 __device__ __forceinline__ void segmentB64Fast(const SegmentHeader &h, const double2 *tt, const double2 *lt,
-                                                 const double2 *pt, const Frame &f, double &H, double &Z)
+                                               const double2 *pt, const Frame &f, int lane, double &H, double &Z)
 {
     H = 0.0;
     Z = 0.0;
@@ -164,9 +167,9 @@ __device__ __forceinline__ void segmentB64Fast(const SegmentHeader &h, const dou
             // F = 2 cB c in [-2 cB, 2 cB]: the roots' arguments d - F and the
             // divisor cC - F (<= both) lie in [cC - 2 cB, max(d1, d2) + 2 cB]
             if (inRange64(cC - 2.0 * fabs(cB), fmax(d1, d2) + 2.0 * fabs(cB)))
-                phiLoopB64<false>(pt, h.n_phi, cA, cB, cC, d1, d2, top, bot, h0, z0);
+                phiLoopB64<false, LANES>(pt, h.n_phi, lane, cA, cB, cC, d1, d2, top, bot, h0, z0);
             else
-                phiLoopB64<true>(pt, h.n_phi, cA, cB, cC, d1, d2, top, bot, h0, z0);
+                phiLoopB64<true, LANES>(pt, h.n_phi, lane, cA, cB, cC, d1, d2, top, bot, h0, z0);
             H += t.y * t.x * h0;
             Z += t.y * z0;
         }
@@ -189,10 +192,10 @@ __device__ __forceinline__ void segmentB64Fast(const SegmentHeader &h, const dou
                     h0 += wg3 * (cB * q.x);
                 };
                 if (inRange64(cD - 2.0 * fabs(cC), cD + 2.0 * fabs(cC)))
-                    for (int k = 0; k < h.n_phi; ++k)
+                    for (int k = lane; k < h.n_phi; k += LANES)
                         node(pt[k], rsqrt64u(cD - 2.0 * cC * pt[k].x));
                 else
-                    for (int k = 0; k < h.n_phi; ++k)
+                    for (int k = lane; k < h.n_phi; k += LANES)
                         node(pt[k], rsqrt64(cD - 2.0 * cC * pt[k].x));
                 const double w = l.y * t.y;
                 H += w * h0;

@@ -532,7 +532,7 @@ __device__ __noinline__ double2 pairB64Fast(const SegmentHeader &h, const double
                                             const double2 *pt, double z, double r)
 {
     double H, Z;
-    segmentB64Fast(h, tt, lt, pt, frameZR(z, r), H, Z);
+    segmentB64Fast(h, tt, lt, pt, frameZR(z, r), 0, H, Z);
     return make_double2(H, Z);
 }
 
