@@ -60,7 +60,7 @@ __device__ __forceinline__ void batchItem(const BatchItem &I, const unsigned cha
     {
         const unsigned char *seg = blob + segs[I.seg_begin + s].offset;
         if (PREC == CCOIL_PRECISION_FP64)
-            integrateSegment64<FIELD, LANES>(seg, px, py, pz, lane, acc);
+            integrateSegment64<FIELD, LANES, true>(seg, px, py, pz, lane, acc);
         else
         {
             const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(seg);
