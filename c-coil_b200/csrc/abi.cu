@@ -174,8 +174,10 @@ int autoLanes64(long long npts, long long pieces, int blocksPerSM)
 // transform, so beyond one wave it keeps kPieceNodes nodes per thread.  FP64 kernel
 // times before and after: A of 24 coils at 1,001 points 310 -> 93 us, B of 64 coils
 // at 4,096 points 1.73 -> 1.07 ms, B of one coil at 37 points 24 -> 8 us; FP32_REFINED
-// A of 128 coils at 200,003 points (2.1 waves whole) 20.4 -> 18.5 ms.
-constexpr long long kFieldWaves = 8, kPieceNodes = 128;
+// A of 128 coils at 200,003 points (2.1 waves whole) 20.4 -> 18.5 ms.  24 waves instead
+// of 8 take 1 to 3 % off calls of 128 coils at 65,536 to 400,000 points (B at 262,144
+// FP32 28.5 -> 28.1, FP64 55.2 -> 54.5 ms), 48 and 96 nothing more.
+constexpr long long kFieldWaves = 24, kPieceNodes = 128;
 FieldSplit fieldSplit(long long npts, int lanes, int nseg, int thickness, long long nodes, int blocksPerSM,
                       bool wholeSegments)
 {

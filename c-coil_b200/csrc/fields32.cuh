@@ -122,18 +122,19 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
         py = points[3 * p + 1];
         pz = points[3 * p + 2];
     }
-    // the gradient's nine sums live in shared memory, one column per thread: in
-    // registers they spill others at 128 (G of 128 coils at 2^17 points: 17.1 ms
-    // against 19.0)
-    constexpr bool kShared = FIELD == CCOIL_FIELD_G;
-    __shared__ double sums[kShared ? W : 1][128];
+    // the sums of the gradient, and of the field where it is not refined, live in
+    // shared memory, one column per thread: in registers they crowd the loops at 128
+    // (128 coils: G at 2^17 points 17.1 ms against 19.0, B at 200,003 points 21.9
+    // against 22.35; the vector potential measured 0.5 % slower this way)
+    constexpr bool kShared = FIELD == CCOIL_FIELD_G || (FIELD == CCOIL_FIELD_B && !REFINE);
+    __shared__ double sums[kShared ? W : 1][kShared ? 128 : 1];
     double acc[W];
 #pragma unroll
     for (int i = 0; i < W; ++i)
     {
         acc[i] = 0.0;
         if (kShared)
-            sums[kShared ? i : 0][threadIdx.x] = 0.0;
+            sums[kShared ? i : 0][kShared ? threadIdx.x : 0] = 0.0;
     }
     // this block's piece of the work (FieldSplit)
     const int piece = blockIdx.y, group = piece / split.parts;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
                 integrateSegment32<FIELD, LANES>(seg, f, lane, c, th);
 #pragma unroll
                 for (int i = 0; i < W; ++i)
-                    sums[kShared ? i : 0][threadIdx.x] += c[i];
+                    sums[kShared ? i : 0][kShared ? threadIdx.x : 0] += c[i];
             }
             else if (!nearPair && !REFINE)
                 integrateSegment32<FIELD, LANES>(seg, f, lane, acc, th);
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
                     for (int i = 0; i < W; ++i)
                     {
                         if (kShared)
-                            sums[kShared ? i : 0][threadIdx.x] += c[i];
+                            sums[kShared ? i : 0][kShared ? threadIdx.x : 0] += c[i];
                         else
                             acc[i] += c[i];
                         dst[i] = c[i];
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
     if (kShared)
 #pragma unroll
         for (int i = 0; i < W; ++i)
-            acc[i] = sums[kShared ? i : 0][threadIdx.x];
+            acc[i] = sums[kShared ? i : 0][kShared ? threadIdx.x : 0];
 #pragma unroll
     for (int off = LANES / 2; off > 0; off /= 2)
 #pragma unroll
@@ -255,12 +256,21 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
     }
 }
 
-// whether a point lies in a segment's near box
+// Whether a point lies in a segment's near box: nearWinding on toCoilFrame, operation
+// for operation, but the radius (a square root) only where the height is in range
 __device__ __forceinline__ bool isNearPair(const unsigned char *blob, const SegmentDesc *segs, int s, double px,
                                            double py, double pz)
 {
     const SegmentHeader &h = *reinterpret_cast<const SegmentHeader *>(blob + segs[s].offset);
-    return nearWinding(h, toCoilFrame(h, px, py, pz));
+    const double *M = h.inv_transform;
+    const double dx = sub(px, h.position[0]), dy = sub(py, h.position[1]), dz = sub(pz, h.position[2]);
+    const double z = add(add(mul(M[6], dx), mul(M[7], dy)), mul(M[8], dz));
+    if (!(z > h.near_lo[1] && z < h.near_hi[1]))
+        return false;
+    const double x = add(add(mul(M[0], dx), mul(M[1], dy)), mul(M[2], dz));
+    const double y = add(add(mul(M[3], dx), mul(M[4], dy)), mul(M[5], dz));
+    const double r = sqr(add(mul(x, x), mul(y, y)));
+    return r > h.near_lo[0] && r < h.near_hi[0];
 }
 
 // Lists the near-field pairs: the pairs of a point in one run of entries, in segment
