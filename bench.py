@@ -76,6 +76,12 @@ def workload_config(a, world):
 # ---------------------------------------------------------------------------
 # reference arm: the reference's own CPU code (oracle/_ref), CPU_MT on all cores
 # ---------------------------------------------------------------------------
+def reference_built():
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    from oracle import Reference
+    return Reference.available()
+
+
 def cpu_reference_rate(a, sample_points):
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     from oracle import Reference
@@ -98,9 +104,7 @@ def reference_arm(a):
     world = int(os.environ.get("WORLD_SIZE", "1"))
     if rank != 0:
         return
-    sys.path.insert(0, os.path.join(ROOT, "oracle"))
-    from oracle import Reference
-    if not Reference.available():
+    if not reference_built():
         print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libccoil_ref.so was not built"}))
         return
     rates = []
@@ -854,20 +858,20 @@ def main():
                 "FT_arrangements_per_s": arr["fp64"]["FT"]["arrangements_per_s"] * world}
         if rates is not None and "fp64" in arr:
             # FP64 pipe model of the arrangement kernels: every (secondary node, primary
-            # node) pair evaluates the reference's A (M) or B (F/T) fast node
+            # node) pair evaluates an A (M) or B (F/T) fast node
             pairs_per_arr = arr["secondary_nodes"] * arr["primary_nodes"]
             roof = {}
             for q, fidx in (("M", 0), ("FT", 1)):
-                am, dv, sq, lg = opcount.OPS_PER_NODE_64[(fidx, True)]
-                slots = pairs_per_arr * (am + dv * rates[0] / rates[1] + sq * rates[0] / rates[2] +
-                                         lg * rates[0] / rates[3]) * a.arrangements
+                slots = pairs_per_arr * opcount.SLOTS_PER_NODE_64[(fidx, True)] * a.arrangements
                 t = arr["fp64"][q]["ms"] * 1e-3
                 roof[q] = {"achieved": 2.0 * slots / t / 1e12, "peak": 2.0 * rates[0] / 1e12, "unit": "TFLOP/s",
                            "frac": slots / t / rates[0]}
             line["arrangements"]["fp64_roofline"] = roof
         # timed launches: M and F/T per precision mode, and per candidate of the 1e-7 configuration
         line["gpu_launches"] += 2 * a.steps * (len(modes) + (2 if "at_1e-7" in arr else 0))
-    if rank == 0 and world == 1 and not a.no_cpu_baseline:
+    if rank == 0 and world == 1 and not a.no_cpu_baseline and not reference_built():
+        line["cpu_baseline"] = {"unavailable": "oracle/_ref/libccoil_ref.so was not built"}
+    elif rank == 0 and world == 1 and not a.no_cpu_baseline:
         rate, cores, dt, desc = cpu_reference_rate(a, a.cpu_sample_points)
         line["cpu_baseline"] = {"value": rate, "unit": UNIT, "cores": cores, "kind": "reference",
                                 "sample": desc, "seconds": dt}
@@ -894,22 +898,28 @@ def ctypes_rates(cc):
 
 
 def field_launches(mode, points, segments, field):
-    """Kernel launches of one field-plan evaluation: FP64 one field kernel; FP32c the field
-    kernel and its near-field FP64 pass, and from 16,384 to 2^30 points also the point
-    ordering (bounds, Morton keys, the radix sort's 6 kernels, gather) and the scatter of
-    the results; FP32_REFINED per chunk of points (contributions of at most 4 GiB, at most
-    2^28 listed pairs) the field kernel, the near-field pass and the selection (count,
-    scan, select) and FP64 pair passes."""
+    """Kernel launches of one field-plan evaluation (one lane per point): the field kernel and,
+    where it is cut into pieces (fewer than 24 waves of 128-point tiles), their sum; in the
+    FP32 modes also the near-field listing and its FP64 pass, and from 16,384 to 2^30 points
+    the point ordering (bounds, Morton keys, the radix sort's 6 kernels, gather) and the
+    scatter of the results; FP32_REFINED per chunk of points (contributions of at most
+    4 GiB, at most 2^28 listed pairs) also the selection (count, scan, select) and FP64 pair
+    passes."""
     mode = int(mode)
+    per_sm = {0: 4, 1: 4, 2: 4, 3: 3}[field] if mode == 0 else {0: 5, 1: 4, 2: 5, 3: 4}[field]
+
+    def sums(n):
+        return 1 if segments > 1 and 24 * 148 * per_sm > -(-n // 128) else 0
+
     if mode == 0:
-        return 1
+        return 1 + sums(points)
     ordering = 10 if (1 << 14) <= points <= (1 << 30) else 0
     if mode == 1:
-        return 2 + ordering
+        return 3 + sums(points) + ordering
     width = 9 if field == 3 else 3
     per_chunk = min((1 << 32) // (segments * width * 8), (1 << 28) // segments)
     chunks = -(-points // max(1, per_chunk))
-    return ordering + 6 * chunks
+    return ordering + (7 + sums(-(-points // chunks))) * chunks
 
 
 def read_profile(field, mode):
