@@ -88,9 +88,15 @@ class _BField(torch.autograd.Function):
 
 def b_field(params, points, precisions=None, precision_factor=5.0):
     """Differentiable group B field at `points` (CUDA tensor) for coil parameter rows `params`."""
+    # the native calls step through the rows and the precisions without their lengths
+    if params.ndim != 2 or params.shape[1] != len(PARAMS):
+        raise ValueError("params must have shape (coils, 9), got %s" % (tuple(params.shape),))
     if precisions is None:
         precisions = precisions_for(params.detach().cpu().numpy(), precision_factor)
-    return _BField.apply(params, points, list(precisions))
+    precisions = list(precisions)
+    if len(precisions) < params.shape[0]:
+        raise ValueError("%d precisions for %d coils" % (len(precisions), params.shape[0]))
+    return _BField.apply(params, points, precisions)
 
 
 def mutual_inductance_position_gradient(primary, secondary, precision_factor=None):

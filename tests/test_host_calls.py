@@ -28,6 +28,22 @@ def test_coils_from_params(ccoil):
     assert lib.ccoil_coils_from_params(q.ctypes.data_as(dp), precs, 9, got) == 1
 
 
+@pytest.mark.parametrize("shape,count", [((2, 8), 2), ((2, 10), 2), ((2, 9), 1), ((9,), 1), ((1, 2, 9), 1)])
+def test_b_field_refuses_rows_and_precisions_of_the_wrong_count(ccoil, monkeypatch, shape, count):
+    # before any native call: those read 9 values and one precision per coil
+    import torch
+    from ccoil_b200 import autograd
+
+    def native():
+        raise AssertionError("native call")
+
+    monkeypatch.setattr(autograd, "lib", native)
+    params = torch.full(shape, 0.1, dtype=torch.float64)
+    precs = [ccoil.PrecisionArguments(1, 1, 1, 10, 3, 2)] * count
+    with pytest.raises(ValueError):
+        autograd.b_field(params, torch.zeros((4, 3), dtype=torch.float64), precs)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["FP64", "FP32_COMPENSATED", "FP32_REFINED"])
 @pytest.mark.parametrize("points", [0, 1, 2730, 2731, 20000])
