@@ -154,7 +154,20 @@ int autoLanes32(long long npts)
     return lanes;
 }
 
-// FP64: points and pieces (segments x thickness nodes) fill the machine first,
+// FP64 in one piece (a captured call, or one without memory for the pieces' sums):
+// only lanes fill the machine.  The rule of the FP32 modes, and 16 or 32 lanes while
+// they take no more than two CTAs per SM.  B captured, 24 coils at 1,001 points: 1, 8
+// and 32 lanes 1,180, 267 and 174 us; at 4,096 points 8, 16 and 32 lanes 313, 326 and
+// 376 us; at 20,000 points 1, 8 and 16 lanes 1,691, 1,117 and 1,269 us.
+int autoLanesOnePiece64(long long npts)
+{
+    int lanes = autoLanes32(npts);
+    while (lanes >= 8 && lanes < 32 && npts * lanes * 2 <= 148LL * 128 * 2)
+        lanes *= 2;
+    return lanes;
+}
+
+// FP64 in pieces: points and pieces (segments x thickness nodes) fill the machine first,
 // because lanes that share a point repeat every thickness node's set-up (8 lanes
 // and 59 angular nodes: a fifth of the work); lanes come in where those are too
 // few for two waves, and to give the warps of a few points something to do
@@ -299,9 +312,18 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
     L.field = plan->field;
     L.precision = plan->precision;
     const int perSM = fieldBlocksPerSM(plan->field, plan->precision);
-    L.lanes = lanes_per_point                              ? lanes_per_point
-              : plan->precision == CCOIL_PRECISION_FP64 ? autoLanes64(point_count, (long long)L.nseg * plan->thickness, perSM)
-                                                        : autoLanes32(point_count);
+    // a captured call runs in one piece: it must not hold an allocation that each
+    // replay would make again
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t captureQuery = cudaStreamIsCapturing(st, &capture);
+    if (captureQuery != cudaSuccess)
+        cudaGetLastError();  // the launches report what is wrong with the stream
+    const bool pieced = L.nseg > 0 && perSM > 0 && captureQuery == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    const bool autoFp64 = lanes_per_point == 0 && plan->precision == CCOIL_PRECISION_FP64;
+    L.lanes = lanes_per_point ? lanes_per_point
+              : !autoFp64     ? autoLanes32(point_count)
+              : pieced        ? autoLanes64(point_count, (long long)L.nseg * plan->thickness, perSM)
+                              : autoLanesOnePiece64(point_count);
     // FP32_REFINED runs in chunks of points whose stored contributions fit
     // kRefineContribBytes and whose pairs fit a list of kRefineListPairs
     const bool refined = plan->precision == CCOIL_PRECISION_FP32_REFINED && L.nseg > 0;
@@ -378,13 +400,10 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
         L.d_out = static_cast<double *>(plan->sortedOut.ptr);
     }
     // the pieces' sums: memory of this call alone (a plan may run on several streams
-    // at once), in the order of the stream.  Without it, or while the stream is
-    // captured (a captured call must not hold an allocation that each replay would
-    // make again), the points are evaluated in one piece
+    // at once), in the order of the stream.  Without it the points are evaluated in
+    // one piece
     void *partial = nullptr;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (L.nseg > 0 && perSM > 0 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
-        capture == cudaStreamCaptureStatusNone)
+    if (pieced)
     {
         const FieldSplit split = fieldSplit(chunk, L.lanes, L.nseg, plan->thickness, plan->nodes, perSM,
                                             refined);
@@ -394,10 +413,12 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
             L.split = split;
             L.d_partial = static_cast<double *>(partial);
         }
-        else
+        else if (pieces > 1)
         {
             partial = nullptr;
             cudaGetLastError();  // an allocation that failed is not this call's error
+            if (autoFp64)
+                L.lanes = autoLanesOnePiece64(point_count);
         }
     }
     int rc = CCOIL_OK;

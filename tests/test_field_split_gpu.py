@@ -51,6 +51,39 @@ def test_pieces_match_captured_call(ccoil, points, field):
     plan.close()
 
 
+@pytest.mark.parametrize("coils,points,lanes", [(24, 300, 32), (24, 1184, 32), (24, 1185, 16), (64, 2368, 16),
+                                                (64, 2369, 8), (8, 18943, 8), (2, 20000, 8), (3, 40000, 4)])
+def test_call_in_one_piece_shares_points_among_lanes(ccoil, coils, points, lanes):
+    """A captured FP64 call, and one whose pieces' allocation fails, run in one piece:
+    then only lanes per point fill the machine.  The lanes order a point's sums, so the
+    automatic choice shows in the bits: those of the expected lane count."""
+    import torch
+    _, c, pts = make(ccoil, coils, points)
+    plan = ccoil.FieldPlan([k.struct() for k in c], 1)
+    x = torch.from_numpy(pts).cuda()
+
+    def captured(n):
+        out = torch.full((points, 3), float("nan"), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            plan(x, lanes=n, out=out)
+        g.replay()
+        torch.cuda.synchronize()
+        return out
+
+    auto, want = captured(0), captured(lanes)
+    assert not torch.equal(captured(1), want)  # the bits do tell lane counts apart
+    assert torch.equal(auto, want)
+    assert ccoil.lib().ccoil_inject_allocation_failures(1) == 0
+    try:
+        failed = plan(x)
+    finally:
+        ccoil.lib().ccoil_inject_allocation_failures(0)
+    assert torch.equal(failed, want)
+    plan.close()
+
+
 @pytest.mark.parametrize("mode", ["FP32_COMPENSATED", "FP32_REFINED"])
 @pytest.mark.parametrize("points", [3, 700, 20011])
 def test_pieces_in_fp32_modes(ccoil, mode, points):
