@@ -1577,7 +1577,8 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     else
         CCOIL_PAIR_LAUNCH(3, true);
 #undef CCOIL_PAIR_LAUNCH
-    if (partial && cudaGetLastError() == cudaSuccess)
+    e = cudaGetLastError();
+    if (e == cudaSuccess && partial)
     {
         const unsigned grid = (unsigned)std::min<long long>((count + 3) / 4, 148LL * 16);
 #define CCOIL_PAIR_REDUCE(W)                                                                                        \
@@ -1592,16 +1593,17 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         else
             CCOIL_PAIR_REDUCE(14);
 #undef CCOIL_PAIR_REDUCE
+        e = cudaGetLastError();
     }
-    if (zPass && cudaGetLastError() == cudaSuccess)
+    if (e == cudaSuccess && zPass)
     {
         // the z-axis pass: one warp per recorded arrangement
         if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE)
             zAxisKernel<0><<<148 * 8, 128, 0, st>>>(dB, dO, zO, primary_count, primP, secP, zL, zN, o);
         else
             zAxisKernel<1><<<148 * 8, 128, 0, st>>>(dB, dO, zO, primary_count, primP, secP, zL, zN, o);
+        e = cudaGetLastError();
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess)
         return cudaFail(e, "pair kernel launch");
     // the call is synchronous, as the reference's: host outputs and the z-axis count
