@@ -504,6 +504,14 @@ struct WarpPose
     int skip;                    // coaxial pair left to the z-axis pass
 };
 
+// pairKernel64's own shared memory for W sums and a team of that many warps, at
+// most; the staged tables come on top
+constexpr size_t pairStaticBytes(int W, int team)
+{
+    const size_t warps = pairThreads(team) / 32;
+    return warps * (sizeof(WarpPose) + 64 * sizeof(int)) + sizeof(double) * (size_t)W * (32 * warps + 2 * warps) + 64;
+}
+
 // FP64 primary quadrature at one secondary node, out of line for the FP32
 // kernel (which takes it only for near-field nodes) so that its register
 // budget does not carry the FP64 integrands.  The point's frame coordinates
@@ -1540,10 +1548,19 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     const size_t smem = (size_t)stagedBytes;
     const auto *zO = zPass ? reinterpret_cast<const long long *>(base + atZOff) : nullptr;
     auto *zL = reinterpret_cast<long long *>(base + atZList);
+    // beyond 48 KiB together with the kernel's own shared memory, the staged tables
+    // have to be asked for
+    const bool beyondDefault = smem + pairStaticBytes(width, team) > size_t(48) * 1024;
 #define CCOIL_PAIR_LAUNCH(Q, F, ...)                                                                                   \
-    pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, pairThreads(team), smem, st>>>(                                          \
-        dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction,  \
-        split, partial)
+    do                                                                                                                 \
+    {                                                                                                                  \
+        if (beyondDefault)                                                                                             \
+            cudaFuncSetAttribute(pairKernel64<Q, F, ##__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                                 CCOIL_PAIR_STAGE_MAX_BYTES);                                                          \
+        pairKernel64<Q, F, ##__VA_ARGS__><<<(unsigned)blocks, pairThreads(team), smem, st>>>(                          \
+            dB, dO, primary_count, primP, secP, count, o, zc, stagedBytes, zO, zL, zN, scratch, scratchNodes, fraction, \
+            split, partial);                                                                                           \
+    } while (0)
     if (quantity == CCOIL_PAIR_MUTUAL_INDUCTANCE && !fp32 && lanes == 8)
         CCOIL_PAIR_LAUNCH(0, false, false, 8);
     else if (quantity == CCOIL_PAIR_FORCE_TORQUE && !fp32 && lanes == 8)

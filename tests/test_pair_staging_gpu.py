@@ -61,3 +61,31 @@ def test_failed_launch_is_an_error_beside_the_z_axis_pass(ccoil, n):
     except ccoil.CCoilError:
         return
     assert np.max(np.abs(got - want) / np.abs(want).max(axis=0)) < 1e-6
+
+
+@pytest.mark.parametrize("quantity,mode", [(0, "FP64"), (0, "FP32_COMPENSATED"), (0, "FP32_REFINED"), (1, "FP64"),
+                                           (1, "FP32_COMPENSATED"), (1, "FP32_REFINED"), (2, "FP64"), (3, "FP64"),
+                                           (3, "FP32_COMPENSATED")])
+@pytest.mark.parametrize("n", [1, 444, 445])
+def test_tables_up_to_the_staging_limit(ccoil, quantity, mode, n):
+    # the bars of test_failed_launch_is_an_error
+    want = arrangements(ccoil, quantity, mode, 1600, n)
+    scale = np.abs(arrangements(ccoil, quantity, mode, 1600, 445)).max(axis=0)
+    for ring in (640, 780, 1000, 1200, 1400, 1480):
+        got = arrangements(ccoil, quantity, mode, ring, n)
+        assert np.max(np.abs(got - want) / scale) < (1e-11 if mode == "FP64" else 1e-5), ring
+
+
+@pytest.mark.parametrize("n", [1, 444])
+@pytest.mark.parametrize("shapes,pf", [(((0.0, 0.0), (0.0, 0.0)), 12.0), (((0.02, 0.05), (0.0, 0.0)), 15.0),
+                                       (((0.0, 0.05), (0.02, 0.0)), 15.0)])
+def test_refined_force_at_high_precision_factors(ccoil, shapes, pf, n):
+    # filament-filament, rectangular-filament, thin-flat: 23 to 28 KB of tables beside
+    # the 12-warp kernel's 27 KB; bar: the refined mode's error of a node against FP64
+    (a, b), (c, d) = shapes
+    P, S = ccoil.Coil(0.1, a, b, 100, 1.0), ccoil.Coil(0.05, c, d, 100, 1.0)
+    s = poses(n)
+    args = (np.zeros((n, 3)), s[:, :3], np.zeros(n), np.zeros(n), s[:, 3], s[:, 4], ccoil.PrecisionFactor(pf))
+    want, got = (ccoil.Coil.compute_all_force_torque_arrangements(P, S, *args, precision_mode=ccoil.PrecisionMode[m])
+                 for m in ("FP64", "FP32_REFINED"))
+    assert np.max(np.abs(got - want) / np.abs(want).max(axis=0)) < 1e-6
