@@ -343,8 +343,8 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
     {
         // near-field work list: room for every (point, segment) pair up to 4 Mi
         // entries (32 MiB; FP32_REFINED: every pair of a chunk, up to
-        // kRefineListPairs); near-field pairs beyond it are integrated in FP64 in
-        // place
+        // kRefineListPairs); with more near-field pairs the near-field pass finds them
+        // itself
         unsigned long long want = (unsigned long long)chunk * (unsigned long long)L.nseg;
         const unsigned long long limit = refined ? kRefineListPairs : (1ULL << 22);
         unsigned long long cap = want < limit ? want : limit;

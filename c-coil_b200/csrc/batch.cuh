@@ -211,18 +211,15 @@ __device__ __forceinline__ void batchNearPoint(const unsigned char *blob, const 
 #pragma unroll
     for (int k = 0; k < W; ++k)
         acc[k] = 0.0;
-    const unsigned long long end = listed ? n : (unsigned long long)segEnd;
-    for (unsigned long long e = listed ? i : (unsigned long long)segBegin; e < end; ++e)
+    NearScan scan = {segBegin, segEnd};
+    for (unsigned long long e = i;; ++e)
     {
-        int s = (int)e;
-        if (listed)
-        {
-            if (work[e].point != (int)p || work[e].segment >> kFieldShift != FIELD)
-                break;
-            s = work[e].segment & ((1 << kFieldShift) - 1);
-        }
-        else if (!isNearPair(blob, segs, s, px, py, pz))
-            continue;
+        if (listed && (e >= n || work[e].point != (int)p || work[e].segment >> kFieldShift != FIELD))
+            break;
+        const int s = listed ? work[e].segment & ((1 << kFieldShift) - 1)
+                             : scan.take(blob, segs, px, py, pz, lane);
+        if (s < 0)
+            break;
         integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
     }
 #pragma unroll

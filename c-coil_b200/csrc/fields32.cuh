@@ -273,6 +273,29 @@ __device__ __forceinline__ bool isNearPair(const unsigned char *blob, const Segm
     return r > h.near_lo[0] && r < h.near_hi[0];
 }
 
+// A warp's walk over a point's near-field segments of [next, end), in order: the
+// lanes test 32 of them at once
+struct NearScan
+{
+    int next, end, first = 0;
+    unsigned found = 0;
+    __device__ __forceinline__ int take(const unsigned char *blob, const SegmentDesc *segs, double px, double py,
+                                        double pz, int lane)
+    {
+        while (found == 0)
+        {
+            if (next >= end)
+                return -1;
+            first = next;
+            next += 32;
+            found = __ballot_sync(0xffffffffu, first + lane < end && isNearPair(blob, segs, first + lane, px, py, pz));
+        }
+        const int s = first + __ffs(found) - 1;
+        found &= found - 1;
+        return s;
+    }
+};
+
 // Lists the near-field pairs: the pairs of a point in one run of entries, in segment
 // order.  It takes every frame transform once more.  LANES (1 or 32) threads per
 // point share its segments.
@@ -352,13 +375,14 @@ __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__re
         for (int k = 0; k < W; ++k)
             acc[k] = 0.0;
         bool any = false;
-        for (unsigned long long e = listed ? i : 0; e < (listed ? n : (unsigned long long)nseg); ++e)
+        NearScan scan = {0, nseg};
+        for (unsigned long long e = i;; ++e)
         {
-            if (listed && work[e].point != (int)p)
+            if (listed && (e >= n || work[e].point != (int)p))
                 break;
-            const int s = listed ? work[e].segment : (int)e;
-            if (!listed && !isNearPair(blob, segs, s, px, py, pz))
-                continue;
+            const int s = listed ? work[e].segment : scan.take(blob, segs, px, py, pz, lane);
+            if (s < 0)
+                break;
             integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
             any = true;
         }

@@ -124,6 +124,28 @@ def test_more_near_pairs_than_the_list_holds(ccoil):
         assert rel_err(out.cpu().numpy(), want).max() < TOL, field
 
 
+@pytest.mark.parametrize("count,n", [(32, 8193), (33, 7944), (77, 3405)])
+def test_overflowing_list_over_groups_of_32_segments(ccoil, count, n):
+    # just more pairs than the allocation-free entry point's list holds (2^18), over
+    # segment counts around whole groups of 32; every second coil is far away
+    import ctypes
+    import torch
+    coils = [ccoil.Coil(0.1, 0.02, 0.05, 10 + i, 1.0 + i, coordinate_position=(0.0, 0.0, 3.0 * (i % 2)))
+             for i in range(2 * count)]
+    g = np.random.default_rng(7)
+    r, phi = g.uniform(0.095, 0.125, n), g.uniform(0.0, 2.0 * np.pi, n)
+    x = torch.from_numpy(np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, n)], axis=1)).cuda()
+    fn = ccoil.lib().ccoil_fields_fp32c_static
+    fn.argtypes = [ctypes.POINTER(ccoil._lib.CoilStruct), ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong,
+                   ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+    structs = (ccoil._lib.CoilStruct * len(coils))(*[c.struct() for c in coils])
+    want = ccoil.FieldPlan(list(structs), 1, ccoil.PrecisionMode.FP32_COMPENSATED)(x).cpu().numpy()
+    out = torch.full((n, 3), float("nan"), dtype=torch.float64, device="cuda")
+    assert fn(structs, len(coils), ctypes.c_void_p(x.data_ptr()), n, 1, ctypes.c_void_p(out.data_ptr()),
+              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert rel_err(out.cpu().numpy(), want).max() < TOL
+
+
 def test_batch_near_pairs_beyond_the_list_and_repeatable(ccoil):
     # one system whose points all lie in the winding boxes of 12 coils: 4.3 million
     # pairs over two fields, more than the batch's list; a second, shorter system
