@@ -341,22 +341,21 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
     }
     if (plan->precision == CCOIL_PRECISION_FP32_COMPENSATED || plan->precision == CCOIL_PRECISION_FP32_REFINED)
     {
-        // near-field work list: room for every (point, segment) pair up to 4 Mi
-        // entries (32 MiB; FP32_REFINED: every pair of a chunk, up to
-        // kRefineListPairs); with more near-field pairs the near-field pass finds them
-        // itself
-        unsigned long long want = (unsigned long long)chunk * (unsigned long long)L.nseg;
-        const unsigned long long limit = refined ? kRefineListPairs : (1ULL << 22);
-        unsigned long long cap = want < limit ? want : limit;
-        if (cap == 0)
-            cap = 1;
-        int rc0 = plan->work.reserve(cap * kNearPairBytes, plan->owner);
+        // near-field work list: room for every (point, segment) pair up to
+        // kNearListPairs (with more near-field pairs the near-field pass finds them
+        // itself; FP32_REFINED's selection: every pair of a chunk, up to
+        // kRefineListPairs), and after it what else the near-field pass needs
+        const unsigned long long want = std::max(1ULL, (unsigned long long)chunk * (unsigned long long)L.nseg);
+        const unsigned long long cap = std::min(want, refined ? kRefineListPairs : kNearListPairs);
+        const unsigned long long near = std::min(want, kNearListPairs);
+        int rc0 = plan->work.reserve(cap * kNearPairBytes + NearScratch::bytes(near, width), plan->owner);
         if (rc0 == CCOIL_OK)
             rc0 = plan->workCount.reserve(sizeof(unsigned long long), plan->owner);
         if (rc0 != CCOIL_OK)
             return rc0;
         L.d_work = plan->work.ptr;
-        L.work_capacity = plan->work.bytes / kNearPairBytes;
+        L.work_capacity = cap;
+        L.near.carve(static_cast<unsigned char *>(plan->work.ptr) + cap * kNearPairBytes, near, width);
         L.d_work_count = static_cast<unsigned long long *>(plan->workCount.ptr);
         L.near_blocks = 148 * 8;
     }

@@ -134,8 +134,11 @@ __global__ void __launch_bounds__(128, batchMinBlocks(PREC)) batchKernel(const u
                                                       const BatchItem *__restrict__ items, int nitems,
                                                       unsigned *__restrict__ next, const double *__restrict__ points,
                                                       double *__restrict__ outA, double *__restrict__ outB,
-                                                      double *__restrict__ outG)
+                                                      double *__restrict__ outG,
+                                                      unsigned long long *__restrict__ workCount)
 {
+    if (PREC != CCOIL_PRECISION_FP64 && blockIdx.x == 0 && threadIdx.x == 0)
+        *workCount = 0;  // the near-field list's counter, for the kernels that follow
     __shared__ int itemIndex;
     __shared__ double sums[PREC == CCOIL_PRECISION_FP64 ? 1 : 9][128];
     for (;;)
@@ -196,51 +199,51 @@ __global__ void __launch_bounds__(128) batchNearListKernel(const unsigned char *
     }
 }
 
-// One warp: the near-field pairs of one point and field, in segment order, FP64,
-// the lanes splitting the angular nodes.  listed: entries [i, ...) of the list up to
-// the point's or field's last; otherwise all segments of [segBegin, segEnd).
+// One warp: near-field pairs of one point and field, FP64, the lanes splitting the
+// angular nodes: a listed pair, whose sums go to contrib, or those of [segBegin,
+// segEnd), in order, which go to out (segment < 0).
 template <int FIELD>
-__device__ __forceinline__ void batchNearPoint(const unsigned char *blob, const SegmentDesc *segs,
-                                               const double *points, double *out, long long p, bool listed,
-                                               const NearPair *work, unsigned long long i, unsigned long long n,
-                                               int segBegin, int segEnd, int lane)
+__device__ __forceinline__ void batchNearPairs(const unsigned char *blob, const SegmentDesc *segs,
+                                               const double *points, long long p, int segment, int segBegin,
+                                               int segEnd, int lane, double *contrib, double *out)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
     const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
-    double acc[W];
-#pragma unroll
-    for (int k = 0; k < W; ++k)
-        acc[k] = 0.0;
+    const bool listed = segment >= 0;
+    double sum = 0.0;
     NearScan scan = {segBegin, segEnd};
-    for (unsigned long long e = i;; ++e)
+    for (int s = listed ? segment : scan.take(blob, segs, px, py, pz, lane); s >= 0;
+         s = listed ? -1 : scan.take(blob, segs, px, py, pz, lane))
     {
-        if (listed && (e >= n || work[e].point != (int)p || work[e].segment >> kFieldShift != FIELD))
-            break;
-        const int s = listed ? work[e].segment & ((1 << kFieldShift) - 1)
-                             : scan.take(blob, segs, px, py, pz, lane);
-        if (s < 0)
-            break;
+        double acc[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            acc[k] = 0.0;
         integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
+#pragma unroll
+        for (int off = 16; off > 0; off /= 2)
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            sum += lane == k ? acc[k] : 0.0;
     }
-#pragma unroll
-    for (int off = 16; off > 0; off /= 2)
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            out[W * p + k] += acc[k];
+    if (listed && lane < W)
+        contrib[lane] = sum;
+    else if (!listed && lane < W && sum != 0.0)
+        out[W * p + lane] += sum;
 }
 
-// Near-field pass of the batched kernel: a warp per run of entries, or, with more
-// pairs than the list holds, per point of each item.
+// Near-field pass of the batched kernel: a warp per entry (batchNearSumKernel adds them
+// up), or, with more pairs than the list holds, a warp per point of each item.
 __global__ void __launch_bounds__(256) batchNearKernel(const unsigned char *__restrict__ blob,
                                                        const SegmentDesc *__restrict__ segs,
                                                        const BatchItem *__restrict__ items, int nitems,
                                                        const double *__restrict__ points, double *__restrict__ outA,
                                                        double *__restrict__ outB, double *__restrict__ outG,
                                                        const NearPair *__restrict__ work,
+                                                       double *__restrict__ contrib, int width,
                                                        unsigned long long workCapacity,
                                                        const unsigned long long *__restrict__ workCount)
 {
@@ -254,14 +257,13 @@ __global__ void __launch_bounds__(256) batchNearKernel(const unsigned char *__re
     for (unsigned long long i = warp; i < end; i += warps)
     {
         long long p;
-        int field, segBegin = 0, segEnd = 0;
+        int field, segment = -1, segBegin = 0, segEnd = 0;
         if (listed)
         {
             const NearPair e = work[i];
             field = e.segment >> kFieldShift;
+            segment = e.segment & ((1 << kFieldShift) - 1);
             p = e.point;
-            if (i > 0 && work[i - 1].point == e.point && work[i - 1].segment >> kFieldShift == field)
-                continue;  // not the first entry of its run
         }
         else
         {
@@ -273,12 +275,41 @@ __global__ void __launch_bounds__(256) batchNearKernel(const unsigned char *__re
             segBegin = I.seg_begin;
             segEnd = I.seg_end;
         }
+        double *entry = contrib + (size_t)width * i;  // listed only
         if (field == CCOIL_FIELD_G)
-            batchNearPoint<CCOIL_FIELD_G>(blob, segs, points, outG, p, listed, work, i, n, segBegin, segEnd, lane);
+            batchNearPairs<CCOIL_FIELD_G>(blob, segs, points, p, segment, segBegin, segEnd, lane, entry, outG);
         else if (field == CCOIL_FIELD_B)
-            batchNearPoint<CCOIL_FIELD_B>(blob, segs, points, outB, p, listed, work, i, n, segBegin, segEnd, lane);
+            batchNearPairs<CCOIL_FIELD_B>(blob, segs, points, p, segment, segBegin, segEnd, lane, entry, outB);
         else
-            batchNearPoint<CCOIL_FIELD_A>(blob, segs, points, outA, p, listed, work, i, n, segBegin, segEnd, lane);
+            batchNearPairs<CCOIL_FIELD_A>(blob, segs, points, p, segment, segBegin, segEnd, lane, entry, outA);
+    }
+}
+
+// Adds the listed pairs' contributions to the outputs, as nearSumKernel
+__global__ void __launch_bounds__(256) batchNearSumKernel(const NearPair *__restrict__ work,
+                                                          unsigned long long workCapacity,
+                                                          const unsigned long long *__restrict__ workCount,
+                                                          const double *__restrict__ contrib, int width,
+                                                          double *__restrict__ outA, double *__restrict__ outB,
+                                                          double *__restrict__ outG)
+{
+    const unsigned long long n = *workCount;
+    if (n > workCapacity)
+        return;
+    const unsigned long long threads = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < n * width; t += threads)
+    {
+        const unsigned long long i = t / width;
+        const int k = (int)(t - i * width);
+        const NearPair e = work[i];
+        const int field = e.segment >> kFieldShift, W = field == CCOIL_FIELD_G ? 9 : 3;
+        auto same = [&](unsigned long long j) {
+            return j < n && work[j].point == e.point && work[j].segment >> kFieldShift == field;
+        };
+        if (k >= W || (i > 0 && same(i - 1)))
+            continue;
+        double *out = field == CCOIL_FIELD_G ? outG : field == CCOIL_FIELD_B ? outB : outA;
+        out[(size_t)W * e.point + k] += nearRunSum(contrib + k, width, i, same);
     }
 }
 
@@ -286,8 +317,6 @@ __global__ void __launch_bounds__(256) batchNearKernel(const unsigned char *__re
 int launchBatchImpl(const BatchLaunch &B, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(B.d_next, 0, sizeof(unsigned), st);
-    if (e == cudaSuccess && B.precision == CCOIL_PRECISION_FP32_COMPENSATED)
-        e = cudaMemsetAsync(B.d_work_count, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return failMessage(CCOIL_ERR_CUDA, cudaGetErrorString(e));
     if (B.nitems == 0)
@@ -296,17 +325,22 @@ int launchBatchImpl(const BatchLaunch &B, cudaStream_t st)
     const BatchItem *items = static_cast<const BatchItem *>(B.d_items);
     if (B.precision == CCOIL_PRECISION_FP64)
         batchKernel<CCOIL_PRECISION_FP64><<<B.grid, 128, 0, st>>>(B.d_blob, B.d_segs, items, B.nitems, B.d_next,
-                                                                     B.d_points, B.d_outA, B.d_outB, B.d_outG);
+                                                                     B.d_points, B.d_outA, B.d_outB, B.d_outG,
+                                                                     nullptr);
     else
         batchKernel<CCOIL_PRECISION_FP32_COMPENSATED><<<B.grid, 128, 0, st>>>(
-            B.d_blob, B.d_segs, items, B.nitems, B.d_next, B.d_points, B.d_outA, B.d_outB, B.d_outG);
+            B.d_blob, B.d_segs, items, B.nitems, B.d_next, B.d_points, B.d_outA, B.d_outB, B.d_outG,
+            B.d_work_count);
     e = cudaGetLastError();
     if (e == cudaSuccess && B.precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {
         batchNearListKernel<<<(unsigned)std::min(B.nitems, 148 * 64), 128, 0, st>>>(
-            B.d_blob, B.d_segs, items, B.nitems, B.fields_mask, B.d_points, work, B.work_capacity, B.d_work_count);
+            B.d_blob, B.d_segs, items, B.nitems, B.fields_mask, B.d_points, work, B.near.capacity, B.d_work_count);
         batchNearKernel<<<148 * 8, 256, 0, st>>>(B.d_blob, B.d_segs, items, B.nitems, B.d_points, B.d_outA, B.d_outB,
-                                                 B.d_outG, work, B.work_capacity, B.d_work_count);
+                                                 B.d_outG, work, B.near.contrib, B.near_width, B.near.capacity,
+                                                 B.d_work_count);
+        batchNearSumKernel<<<148 * 8, 256, 0, st>>>(work, B.near.capacity, B.d_work_count, B.near.contrib,
+                                                    B.near_width, B.d_outA, B.d_outB, B.d_outG);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? CCOIL_OK : failMessage(CCOIL_ERR_CUDA, cudaGetErrorString(e));

@@ -154,7 +154,9 @@ BatchLaunch launchOf(ccoil_batch_plan *P, const double *pts, double *a, double *
     if (P->precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {
         B.d_work = P->work.p;
-        B.work_capacity = P->work.n / kNearPairBytes;
+        B.near_width = P->fields_mask & (1 << CCOIL_FIELD_G) ? 9 : 3;
+        B.near.carve(static_cast<unsigned char *>(P->work.p) + kNearPairBytes * kBatchListPairs, kBatchListPairs,
+                     B.near_width);
         B.d_work_count = static_cast<unsigned long long *>(P->workCount.p);
     }
     return B;
@@ -250,7 +252,8 @@ int ccoil_batch_plan_create(const ccoil_coil_t *coils, const int *system_coil_of
         rc = P->next.reserve(256);
     if (rc == CCOIL_OK && precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {
-        rc = P->work.reserve(kNearPairBytes * (1u << 22));
+        rc = P->work.reserve(kNearPairBytes * kBatchListPairs +
+                             NearScratch::bytes(kBatchListPairs, fields_mask & (1 << CCOIL_FIELD_G) ? 9 : 3));
         if (rc == CCOIL_OK)
             rc = P->workCount.reserve(sizeof(unsigned long long));
     }

@@ -166,6 +166,34 @@ struct FieldSplit
     int groups = 1, parts = 1;
 };
 
+// Near-field pairs that are listed and evaluated a warp each (with more, the near-field
+// pass finds them itself, a warp per point): besides the list, room for the contribution
+// of every entry (w values) and, for calls of up to kNearRunPairs (point, segment) pairs,
+// its run.
+constexpr size_t kNearPairBytes = 8, kNearRunBytes = 12;
+constexpr unsigned long long kNearRunPairs = 1ULL << 15;
+struct NearScratch
+{
+    unsigned long long capacity = 0;
+    double *contrib = nullptr;
+    void *runs = nullptr;
+    static constexpr size_t bytes(unsigned long long pairs, int w)
+    {
+        return sizeof(double) * w * (size_t)pairs + kNearRunBytes * (size_t)(pairs < kNearRunPairs ? pairs : kNearRunPairs);
+    }
+    void carve(void *base, unsigned long long pairs, int w)
+    {
+        capacity = pairs;
+        contrib = static_cast<double *>(base);
+        runs = contrib + (size_t)pairs * w;
+    }
+};
+// Plans list at most this many: 8 MiB of list, 24 MiB of contributions (72 MiB for the
+// gradient).  The benchmark's groups have 0.07 to 0.4 pairs per point; with more than
+// these a warp per point fills the machine, unless fewer than 9,472 points lie in more
+// than 110 boxes each.  Batch plans a quarter.
+constexpr unsigned long long kNearListPairs = 1ULL << 20, kBatchListPairs = 1ULL << 18;
+
 // kernels (fields.cu)
 struct FieldLaunch
 {
@@ -183,6 +211,7 @@ struct FieldLaunch
     unsigned long long work_capacity = 0;
     unsigned long long *d_work_count = nullptr;
     int near_blocks = 0;                    // grid of the near-field pass
+    NearScratch near;
     FieldSplit split;
     double *d_partial = nullptr;
     // FP32_REFINED: every (point, segment) FP32 contribution whose norm exceeds
@@ -196,7 +225,6 @@ struct FieldLaunch
     unsigned long long *d_refine_segs = nullptr;  // nseg counters (scratch)
     unsigned long long *d_refined_total = nullptr;
 };
-constexpr size_t kNearPairBytes = 8;
 // default fraction of FP32_REFINED (ccoil_set_refine_fraction): on the 128-coil
 // benchmark group it re-evaluates about 12 % of the (point, coil) pairs in FP64
 // and brings the maximum relative error of A and B below 1e-7
@@ -242,9 +270,10 @@ struct BatchLaunch
     int precision;
     int fields_mask;  // bits 1 << CCOIL_FIELD_A, _B, _G
     int grid;
-    void *d_work = nullptr;
-    unsigned long long work_capacity = 0;
+    void *d_work = nullptr;    // NearPair[near.capacity]
     unsigned long long *d_work_count = nullptr;
+    NearScratch near;          // near_width values per pair
+    int near_width = 0;        // 9 with the gradient among the fields, else 3
 };
 constexpr size_t kBatchItemBytes = 32;
 

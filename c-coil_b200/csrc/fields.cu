@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(32 * ROWS) sumPiecesKernel(const double *__res
 }
 
 #include "fields32.cuh"
+static_assert(sizeof(NearPair) == kNearPairBytes && sizeof(NearRun) == kNearRunBytes, "near-field list layout");
 #include "batch.cuh"
 
 template <int FIELD>
@@ -287,7 +288,8 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
     {
 #define CCOIL_LAUNCH32(N, R)                                                                                      \
     fieldsKernel32<FIELD, N, R><<<grid, threads, smem, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts,     \
-                                                             L.d_out, R ? L.d_contrib : nullptr, L.split, partial)
+                                                             L.d_out, R ? L.d_contrib : nullptr, L.split, partial,     \
+                                                             L.d_work_count)
 #define CCOIL_CASE(N, REFINING)                                                                                   \
     case N:                                                                                                       \
         if (refine)                                                                                               \
@@ -324,14 +326,22 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
     // host synchronisation is needed between the passes
     // few points and many segments: a warp per point (84 segments, 2,797 points: 10 us
     // against 70)
+    // With few pairs the near-field kernel adds up each point's itself, which saves a
+    // launch (24 coils, 300 points: 1.6 of 45 us) but costs every warp a fence and an
+    // atomic (70 thin coils, 30,000 points, 420,000 pairs: 1,546 against 1,200 us)
+    const bool fewPairs = (unsigned long long)L.npts * L.nseg <= kNearRunPairs;
+    NearRun *runs = fewPairs ? reinterpret_cast<NearRun *>(L.near.runs) : nullptr;
     if (L.nseg >= 16 && L.npts <= (1 << 15))
         nearListKernel<32><<<(unsigned)((L.npts + 7) / 8), 256, 0, st>>>(
-            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, L.work_capacity, L.d_work_count);
+            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, runs, L.near.capacity, L.d_work_count);
     else
         nearListKernel<1><<<(unsigned)((L.npts + 255) / 256), 256, 0, st>>>(
-            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, L.work_capacity, L.d_work_count);
+            L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, work, runs, L.near.capacity, L.d_work_count);
     nearFieldKernel<FIELD><<<L.near_blocks, 256, 0, st>>>(L.d_blob, L.d_segs, L.nseg, L.d_points, L.npts, L.d_out,
-                                                          work, L.work_capacity, L.d_work_count);
+                                                          work, runs, L.near.contrib, L.near.capacity, L.d_work_count);
+    if (!fewPairs)
+        nearSumKernel<FIELD == CCOIL_FIELD_G ? 9 : 3><<<L.near_blocks, 256, 0, st>>>(
+            work, L.near.capacity, L.d_work_count, L.near.contrib, L.d_out);
     e = cudaGetLastError();
     if (e != cudaSuccess || !refine)
         return e;
@@ -372,9 +382,11 @@ int launchFields(const FieldLaunch &L, void *stream)
     {
         if (L.npts > 2147483647LL)
             return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "FP32_COMPENSATED supports at most 2^31-1 points per call");
-        if (!L.d_work || !L.d_work_count)
+        if (!L.d_work || !L.d_work_count || !L.near.runs || !L.near.contrib)
             return failMessage(CCOIL_ERR_INVALID_ARGUMENT, "FP32_COMPENSATED needs a near-field work list");
-        e = cudaMemsetAsync(L.d_work_count, 0, sizeof(unsigned long long), st);
+        e = clearsNearCount(L.field, L.precision == CCOIL_PRECISION_FP32_REFINED)
+                ? cudaSuccess
+                : cudaMemsetAsync(L.d_work_count, 0, sizeof(unsigned long long), st);
         if (e != cudaSuccess)
             return failMessage(CCOIL_ERR_CUDA, cudaGetErrorString(e));
     }

@@ -6,9 +6,10 @@
 // left out by the FP32 loop.  A second kernel lists such (point, segment) pairs,
 // a point's pairs next to each other and in segment order, and a third evaluates
 // them with the FP64 integrands, so warps never diverge between the two paths.
-// One warp adds all pairs of a point, in order: results repeat exactly however the
-// FP32 pass is cut into pieces.  If the list is too short for all pairs, the third
-// kernel finds and evaluates them itself.
+// A warp evaluates a pair, and a point's pairs are added in order: results repeat
+// exactly however the FP32 pass is cut into pieces, and a point that lies in many
+// windings' boxes does not wait for one warp.  If the list is too short for all pairs,
+// the third kernel finds them itself, a warp per point.
 //
 // FP32_REFINED.  The FP32 kernel also stores every (point, segment)
 // contribution; once the point's total is known, a selection kernel removes
@@ -54,6 +55,12 @@ struct NearPair
     int point;
     int segment;
 };
+// Its run, where the third kernel adds up the runs itself: the entries of one point, and,
+// with the run's first entry, how many of them have been evaluated
+struct NearRun
+{
+    int first, count, done;
+};
 
 // CTAs per SM the register allocation targets (128 threads each): the packed
 // FP32 integrands hold two mirror pairs per value, and these are the highest
@@ -82,6 +89,11 @@ constexpr int fp32MinBlocks(int field)
 #define CCOIL_FP32_STAGE 0
 #endif
 
+// Whether the field kernel clears the near-field list's counter, which saves a launch (2
+// of 24 us for 2 coils at 37 points).  Not the refined gradient's: the compiler then gives
+// its loops other registers (128 coils at 65,536 points 9.89 -> 10.05 ms).
+constexpr bool clearsNearCount(int field, bool refine) { return !(refine && field == CCOIL_FIELD_G); }
+
 // REFINE (FP32_REFINED): every (point, segment) contribution is also written
 // to contrib, segment-major ([segment][point][W], so a warp's stores for one
 // segment are contiguous), near-field pairs as zeros (they are FP64 already)
@@ -91,12 +103,15 @@ __global__ void __launch_bounds__(128, fp32MinBlocks(FIELD)) fieldsKernel32(cons
                                                       const double *__restrict__ points, long long npts,
                                                       double *__restrict__ out, double *__restrict__ contrib,
                                                       FieldSplit split,
-                                                      double *__restrict__ partial)
+                                                      double *__restrict__ partial,
+                                                      unsigned long long *__restrict__ workCount)
 {
     constexpr int W = FIELD == CCOIL_FIELD_G ? 9 : 3;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[kSegmentStages];
     __shared__ int timedOut;
+    if (clearsNearCount(FIELD, REFINE) && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        *workCount = 0;
 
     const int lane = threadIdx.x % LANES;
     const long long p = (long long)blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
@@ -297,13 +312,14 @@ struct NearScan
 };
 
 // Lists the near-field pairs: the pairs of a point in one run of entries, in segment
-// order.  It takes every frame transform once more.  LANES (1 or 32) threads per
-// point share its segments.
+// order, and beside every entry its run (runs != null).  It takes every frame transform
+// once more.
+// LANES (1 or 32) threads per point share its segments.
 template <int LANES>
 __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__restrict__ blob,
                                                          const SegmentDesc *__restrict__ segs, int nseg,
                                                          const double *__restrict__ points, long long npts,
-                                                         NearPair *__restrict__ work,
+                                                         NearPair *__restrict__ work, NearRun *__restrict__ runs,
                                                          unsigned long long workCapacity,
                                                          unsigned long long *__restrict__ workCount)
 {
@@ -330,6 +346,7 @@ __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__
     unsigned long long slot = lane == 0 ? atomicAdd(workCount, (unsigned long long)count) : 0ull;
     if (LANES > 1)
         slot = __shfl_sync(0xffffffffu, slot, 0);
+    const NearRun run = {(int)slot, count, 0};  // not read if the list is too short
     for (int s0 = first / LANES * LANES; s0 < nseg && slot < workCapacity; s0 += LANES)
     {
         const bool near = s0 + lane < nseg && isNearPair(blob, segs, s0 + lane, px, py, pz);
@@ -339,20 +356,83 @@ __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__
         {
             work[at].point = (int)p;
             work[at].segment = s0 + lane;
+            if (runs)
+                runs[at] = run;
         }
         slot += __popc(before);
     }
 }
 
-// Evaluates the near-field pairs: one warp per point's run of entries, the FP64
-// integrands read from the segment blob in global memory, the lanes splitting the
-// angular nodes; the warp alone adds to the point's output.  With more pairs than
-// the list holds, the warps go over all points instead.
+// One value of one point: the sum of its contributions, entries first, first + 1, ... of
+// the list while in(entry) holds, eight loaded at a time (a run of 64 is a chain of 8
+// loads) and added in order.
+template <typename In>
+__device__ __forceinline__ double nearRunSum(const double *contrib, int stride, unsigned long long first, In in)
+{
+    double sum = 0.0;
+    for (bool more = true; more; first += 8)
+    {
+        double v[8];
+        bool is[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+            is[j] = in(first + j);
+            v[j] = is[j] ? __ldcg(contrib + (size_t)stride * (first + j)) : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+            more = more && is[j];
+            if (more)
+                sum += v[j];
+        }
+    }
+    return sum;
+}
+
+// A warp's sums of listed pair i (every lane has them) on their way to out: the warp
+// that brings the last pair of a run adds the run, whichever warp that is.
+template <int W>
+__device__ __forceinline__ void addListedPair(const double *acc, unsigned long long i, NearRun *runs, double *contrib,
+                                              double *out, int lane)
+{
+    const int first = runs[i].first, count = runs[i].count;
+    if (count == 1)
+    {
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                out[k] += acc[k];
+        return;
+    }
+    int before = 0;
+    if (lane == 0)
+    {
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            __stcg(&contrib[(size_t)W * i + k], acc[k]);
+        __threadfence();
+        before = atomicAdd(&runs[first].done, 1);
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) != count - 1)
+        return;
+    __syncwarp();
+    __threadfence();
+    if (lane < W)
+        out[lane] += nearRunSum(contrib + lane, W, first, [&](unsigned long long e) { return e < first + count; });
+}
+
+// Evaluates the near-field pairs, the FP64 integrands read from the segment blob in
+// global memory, the lanes of a warp splitting the angular nodes: a warp per entry of
+// the list, its sums to contrib[entry], or, with more pairs than it holds, a warp per
+// point of all points.  runs != null: this kernel adds the runs; else nearSumKernel does.
 template <int FIELD>
 __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__restrict__ blob,
                                                        const SegmentDesc *__restrict__ segs, int nseg,
                                                        const double *__restrict__ points, long long npts,
                                                        double *__restrict__ out, const NearPair *__restrict__ work,
+                                                       NearRun *runs, double *contrib,
                                                        unsigned long long workCapacity,
                                                        const unsigned long long *__restrict__ workCount)
 {
@@ -362,43 +442,61 @@ __global__ void __launch_bounds__(256) nearFieldKernel(const unsigned char *__re
     const int lane = threadIdx.x % 32;
     const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const unsigned long long warps = (unsigned long long)gridDim.x * blockDim.x / 32;
-    // entry (listed) or point i; a point's entries are consecutive
     const unsigned long long end = listed ? n : (unsigned long long)npts;
     for (unsigned long long i = warp; i < end; i += warps)
     {
         const long long p = listed ? work[i].point : (long long)i;
-        if (listed && i > 0 && work[i - 1].point == (int)p)
-            continue;  // not the first entry of its run
         const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
-        double acc[W];
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-            acc[k] = 0.0;
-        bool any = false;
+        double sum = 0.0;  // lane k of a warp per point: value k
         NearScan scan = {0, nseg};
-        for (unsigned long long e = i;; ++e)
+        for (int s = listed ? work[i].segment : scan.take(blob, segs, px, py, pz, lane); s >= 0;
+             s = listed ? -1 : scan.take(blob, segs, px, py, pz, lane))
         {
-            if (listed && (e >= n || work[e].point != (int)p))
-                break;
-            const int s = listed ? work[e].segment : scan.take(blob, segs, px, py, pz, lane);
-            if (s < 0)
-                break;
+            double acc[W];
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                acc[k] = 0.0;
             integrateSegment64<FIELD, 32>(blob + segs[s].offset, px, py, pz, lane, acc);
-            any = true;
+            // pair by pair, so that a point's sum is the same either way
+#pragma unroll
+            for (int off = 16; off > 0; off /= 2)
+#pragma unroll
+                for (int k = 0; k < W; ++k)
+                    acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+            if (listed && runs)
+                addListedPair<W>(acc, i, runs, contrib, out + W * p, lane);
+            else
+#pragma unroll
+                for (int k = 0; k < W; ++k)
+                    sum += lane == k ? acc[k] : 0.0;
         }
-        if (!any)
+        if (listed && !runs && lane < W)
+            contrib[W * i + lane] = sum;
+        else if (!listed && lane < W && sum != 0.0)
+            out[W * p + lane] += sum;
+    }
+}
+
+// Adds the listed pairs' contributions to the output: a thread per entry and value,
+// those of a run's first entry take the run.
+template <int W>
+__global__ void __launch_bounds__(256) nearSumKernel(const NearPair *__restrict__ work,
+                                                     unsigned long long workCapacity,
+                                                     const unsigned long long *__restrict__ workCount,
+                                                     const double *__restrict__ contrib, double *__restrict__ out)
+{
+    const unsigned long long n = *workCount;
+    if (n > workCapacity)
+        return;
+    const unsigned long long threads = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < n * W; t += threads)
+    {
+        const unsigned long long i = t / W;
+        const int k = (int)(t - i * W), p = work[i].point;
+        if (i > 0 && work[i - 1].point == p)
             continue;
-#pragma unroll
-        for (int off = 16; off > 0; off /= 2)
-#pragma unroll
-            for (int k = 0; k < W; ++k)
-                acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        if (lane == 0)
-        {
-#pragma unroll
-            for (int k = 0; k < W; ++k)
-                out[W * p + k] += acc[k];
-        }
+        out[(size_t)W * p + k] +=
+            nearRunSum(contrib + k, W, i, [&](unsigned long long e) { return e < n && work[e].point == p; });
     }
 }
 

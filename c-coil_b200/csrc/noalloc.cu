@@ -25,10 +25,10 @@ namespace
 {
 constexpr size_t kStaticBlobBytes = 1u << 20;        // node tables
 constexpr int kStaticMaxSegments = 8192;              // segment descriptors (128 KiB)
-constexpr size_t kStaticWorkEntries = 1u << 18;       // near-field work list (2 MiB)
+constexpr size_t kStaticWorkBytes = 2u << 20;         // near-field work list, its runs and contributions
 constexpr size_t kOffSegs = kStaticBlobBytes;
 constexpr size_t kOffWork = kOffSegs + sizeof(SegmentDesc) * kStaticMaxSegments;
-constexpr size_t kOffCount = kOffWork + kNearPairBytes * kStaticWorkEntries;
+constexpr size_t kOffCount = kOffWork + kStaticWorkBytes;
 constexpr size_t kStaticScratchBytes = kOffCount + 256;
 constexpr int kMaxDevices = 64;
 
@@ -179,9 +179,11 @@ extern "C" int ccoil_fields_fp32c_static(const ccoil_coil_t *coils, int coil_cou
     L.field = field;
     L.precision = CCOIL_PRECISION_FP32_COMPENSATED;
     L.lanes = point_count >= 148LL * 1024 ? 1 : point_count >= 148LL * 512 ? 2 : point_count >= 148LL * 256 ? 4 : 8;
+    // room for 53,248 near-field pairs, for the gradient 21,299
     L.d_work = scratch + kOffWork;
-    L.work_capacity = kStaticWorkEntries;
-    L.d_work_count = reinterpret_cast<unsigned long long *>(scratch + kOffCount);  // zeroed by launchFields
+    L.work_capacity = (kStaticWorkBytes - kNearRunBytes * kNearRunPairs) / (kNearPairBytes + sizeof(double) * width);
+    L.d_work_count = reinterpret_cast<unsigned long long *>(scratch + kOffCount);  // zeroed by the field kernel
+    L.near.carve(scratch + kOffWork + kNearPairBytes * L.work_capacity, L.work_capacity, width);
     L.near_blocks = 148 * 8;
     return launchFields(L, stream);
 }
