@@ -311,10 +311,57 @@ struct NearScan
     }
 };
 
+// How many of the segments [begin, end) have the point in their near box, and the first
+// one; LANES (1 or 32) threads share them
+template <int LANES>
+__device__ __forceinline__ int countNear(const unsigned char *blob, const SegmentDesc *segs, int begin, int end,
+                                         double px, double py, double pz, int lane, int &first)
+{
+    int count = 0;
+    first = end;
+#pragma unroll 2
+    for (int s = begin + lane; s < end; s += LANES)
+        if (isNearPair(blob, segs, s, px, py, pz))
+        {
+            first = min(first, s);
+            ++count;
+        }
+    if (LANES > 1)
+    {
+        count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
+        first = (int)__reduce_min_sync(0xffffffffu, (unsigned)first);
+    }
+    return count;
+}
+
+// Their entries, in segment order from slot on, with `tag` in the segment's top bits, and
+// beside every entry its run (runs != null)
+template <int LANES>
+__device__ __forceinline__ void listNear(const unsigned char *blob, const SegmentDesc *segs, int first, int end,
+                                         double px, double py, double pz, long long p, int lane, int tag,
+                                         unsigned long long slot, int count, NearPair *work, NearRun *runs,
+                                         unsigned long long workCapacity)
+{
+    const NearRun run = {(int)slot, count, 0};  // not read if the list is too short
+    for (int s0 = first; s0 < end && slot < workCapacity; s0 += LANES)
+    {
+        const bool near = s0 + lane < end && isNearPair(blob, segs, s0 + lane, px, py, pz);
+        const unsigned before = LANES > 1 ? __ballot_sync(0xffffffffu, near) : (near ? 1u : 0u);
+        const unsigned long long at = slot + __popc(before & ((1u << lane) - 1u));
+        if (near && at < workCapacity)
+        {
+            work[at].point = (int)p;
+            work[at].segment = (s0 + lane) | tag;
+            if (runs)
+                runs[at] = run;
+        }
+        slot += __popc(before);
+    }
+}
+
 // Lists the near-field pairs: the pairs of a point in one run of entries, in segment
-// order, and beside every entry its run (runs != null).  It takes every frame transform
-// once more.
-// LANES (1 or 32) threads per point share its segments.
+// order.  It takes every frame transform once more.  LANES (1 or 32) threads per point
+// share its segments.
 template <int LANES>
 __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__restrict__ blob,
                                                          const SegmentDesc *__restrict__ segs, int nseg,
@@ -328,39 +375,14 @@ __global__ void __launch_bounds__(256, 4) nearListKernel(const unsigned char *__
     if (p >= npts)
         return;
     const double px = points[3 * p], py = points[3 * p + 1], pz = points[3 * p + 2];
-    int count = 0, first = nseg;
-#pragma unroll 2
-    for (int s = lane; s < nseg; s += LANES)
-        if (isNearPair(blob, segs, s, px, py, pz))
-        {
-            first = min(first, s);
-            ++count;
-        }
-    if (LANES > 1)
-    {
-        count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
-        first = (int)__reduce_min_sync(0xffffffffu, (unsigned)first);
-    }
+    int first;
+    const int count = countNear<LANES>(blob, segs, 0, nseg, px, py, pz, lane, first);
     if (count == 0)
         return;
     unsigned long long slot = lane == 0 ? atomicAdd(workCount, (unsigned long long)count) : 0ull;
     if (LANES > 1)
         slot = __shfl_sync(0xffffffffu, slot, 0);
-    const NearRun run = {(int)slot, count, 0};  // not read if the list is too short
-    for (int s0 = first / LANES * LANES; s0 < nseg && slot < workCapacity; s0 += LANES)
-    {
-        const bool near = s0 + lane < nseg && isNearPair(blob, segs, s0 + lane, px, py, pz);
-        const unsigned before = LANES > 1 ? __ballot_sync(0xffffffffu, near) : (near ? 1u : 0u);
-        const unsigned long long at = slot + __popc(before & ((1u << lane) - 1u));
-        if (near && at < workCapacity)
-        {
-            work[at].point = (int)p;
-            work[at].segment = s0 + lane;
-            if (runs)
-                runs[at] = run;
-        }
-        slot += __popc(before);
-    }
+    listNear<LANES>(blob, segs, first, nseg, px, py, pz, p, lane, 0, slot, count, work, runs, workCapacity);
 }
 
 // One value of one point: the sum of its contributions, entries first, first + 1, ... of
