@@ -180,7 +180,10 @@ __device__ __forceinline__ ADSums phiLoopAD64(const double2 *pt, int n, int lane
         double n1, e1, n2, e2;
         node(q, n1, e1);
         node(qm, n2, e2);
-        S.v = fma(0.5 * (q.y * q.x - qm.y * qm.x), logRatio64t<CHECKED>(n1 * e2, e1 * n2), S.v);
+        // (outside the range the products of four lengths would leave that of FP64)
+        const double lg = CHECKED ? logRatio64t<CHECKED>(n1, e1) - logRatio64t<CHECKED>(n2, e2)
+                                  : logRatio64t<CHECKED>(n1 * e2, e1 * n2);
+        S.v = fma(0.5 * (q.y * q.x - qm.y * qm.x), lg, S.v);
     }
     if ((n & 1) && lane == 0)
     {

@@ -99,3 +99,38 @@ def test_adjoint_sums_over_points(ccoil, points):
     whole, half = grad(pts), points // 2
     parts = grad(pts[:half]) + grad(pts[half:])
     assert np.max(np.abs(parts - whole) / np.abs(whole).max(axis=0)) < 1e-12
+
+
+@pytest.mark.parametrize("shape,scale",
+                         [(k, s) for k in ((0.02, 0.1), (0.0, 0.1), (0.03, 0.0))
+                          for s in (1e10, 3e17, 1e21, 1e40, 1e76, 1e80, 1e120)
+                          # the length nodes' 1 / distance^3 leaves FP64's range at 1e103
+                          if not (k[1] == 0.0 and s == 1e120)])
+@pytest.mark.parametrize("quantity", [2, 3])
+def test_pair_gradient_is_scale_invariant(ccoil, scale, shape, quantity):
+    """M grows as a length: with every length scaled by s, its derivatives by lengths stay
+    and those by angles (and M) scale by s.  One pose lies inside the winding.  Bar 1e-11
+    of each column's scale, as for the adjoint above."""
+    from ccoil_b200 import coil as C
+    g = np.random.default_rng(44)
+    v = g.normal(size=(7, 3))
+    v *= g.uniform(0.15, 0.4, (7, 1)) / np.linalg.norm(v, axis=1, keepdims=True)
+    v[0] = [0.001, 0.002, 0.003]
+    turns = g.uniform(0.1, 3.0, (7, 4))
+    a, b = shape
+    pa, sa = ccoil.Coil._pair_args(ccoil.Coil(0.1, a, b, 100, 1.0), ccoil.Coil(0.05, 0.0, 0.05, 100, 1.0), 3.0)
+
+    def values(s):
+        P, S = ccoil.Coil(0.1 * s, a * s, b * s, 100, 1.0), ccoil.Coil(0.05 * s, 0.0, 0.05 * s, 100, 1.0)
+        out = C._pair_arrangements([P.struct(pa)], S.struct(sa), [sa.to_struct()],
+                                   np.column_stack([np.zeros((7, 3)), turns[:, :2]]),
+                                   np.column_stack([v * s, turns[:, 2:]]), quantity)[0].copy()
+        if quantity == 3:
+            out[:, [0, 4, 5, 12, 13]] /= s
+            # a zero dimension is 1e-25 R at any scale
+            out[:, [k for k, d in ((2, a), (3, b), (7, 0.0)) if d == 0.0]] = 0.0
+        return out
+
+    want = values(1.0)
+    bar = 1e-11 * np.abs(want).max(axis=0)
+    assert np.all(np.abs(values(scale) - want) <= bar)
