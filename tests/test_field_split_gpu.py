@@ -233,3 +233,20 @@ def test_pairs_of_one_point_run_side_by_side(ccoil):
     far, near = time(0.0, 0.0, 0.016), time(0.105, 0.0, 0.016)
     plan.close()
     assert near < 4.0 * far, (near, far)
+
+
+def test_batch_overflow_with_segments_shared_in_a_warp(ccoil):
+    # 33 coils in one place: listed a warp per point; 4,100 points give 270,600 pairs over
+    # two fields, more than the list's 2^18, and 3,900 points 257,400, fewer.  Every pair is
+    # FP64, so the plan's sums, in the same order
+    coils = [ccoil.Coil(0.1, 0.02, 0.05, 10 + i, 1.0 + i) for i in range(33)]
+    g = np.random.default_rng(9)
+    for n in (3900, 4100):
+        r, phi = g.uniform(0.095, 0.125, n), g.uniform(0.0, 2.0 * np.pi, n)
+        pts = np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, n)], axis=1)
+        batch = ccoil.BatchPlan([(coils, pts)], fields=("A", "B"), precision=ccoil.PrecisionMode.FP32_COMPENSATED)
+        got = batch.run()
+        for f, field in (("A", 0), ("B", 1)):
+            want = ccoil.FieldPlan([c.struct() for c in coils], field, ccoil.PrecisionMode.FP32_COMPENSATED)(pts)
+            assert rel_err(got[f].cpu().numpy(), want).max() < TOL, (f, n)
+        batch.close()
