@@ -80,6 +80,7 @@ __device__ __forceinline__ double div64u(double n, double d)
 //   div64u   (above) likewise 0.5 ulp + 2^-26 ulp: 2 of 7.3e9 differed.
 // FP64-pipe operations: root64 8, root64n 6, a reciprocal 2, a quotient 3, div64u
 // 5, where the compiler's IEEE root takes 13 and its division 8.
+// ccoil_eval_integrand_op exposes them (tests/test_log64_gpu.py).
 struct Root64
 {
     double y;  // 1 / sqrt(x), to about one ulp (root64) or 2^-38 (root64n)

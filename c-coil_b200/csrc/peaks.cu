@@ -143,6 +143,21 @@ __global__ void fp64OpKernel(int op, const double *__restrict__ a, const double 
         out[i] = op == 0 ? rsqrt64u(a[i]) : op == 1 ? sqrt64u(a[i]) : op == 2 ? div64u(a[i], b[i]) : logRatio64(a[i], b[i]);
 }
 
+// The FP64 integrands' forms: op 0: sqrt(a), 1: 1 / sqrt(a) (root64, reciprocal64),
+// 2 and 3: the same from root64n, 4: a / sqrt(b) (root64n, quotient64), 5: 1 / a (rcp64u)
+__global__ void integrandOpKernel(int op, const double *__restrict__ a, const double *__restrict__ b,
+                                  double *__restrict__ out, long long n)
+{
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    {
+        const Root64 r = op < 2 ? root64(a[i]) : root64n(op == 4 ? b[i] : a[i]);
+        out[i] = op == 0 || op == 2   ? r.s
+                 : op == 1 || op == 3 ? reciprocal64(r.s, r.y)
+                 : op == 4            ? quotient64(a[i], r.s, r.y)
+                                      : rcp64u(a[i]);
+    }
+}
+
 template <typename Launch>
 float timeIt(Launch launch)
 {
@@ -277,5 +292,14 @@ extern "C" int ccoil_eval_fp64_op(int op, const double *a, const double *b, doub
         return fail(CCOIL_ERR_INVALID_ARGUMENT, "op must be 0 (rsqrt), 1 (sqrt), 2 (divide) or 3 (log of a ratio)");
     return evalElementwise(n, a && out && (op < 2 || b), stream, [&](unsigned grid, cudaStream_t st) {
         fp64OpKernel<<<grid, 256, 0, st>>>(op, a, b, out, n);
+    });
+}
+
+extern "C" int ccoil_eval_integrand_op(int op, const double *a, const double *b, double *out, long long n, void *stream)
+{
+    if (op < 0 || op > 5)
+        return fail(CCOIL_ERR_INVALID_ARGUMENT, "op must be 0 to 5");
+    return evalElementwise(n, a && out && (op != 4 || b), stream, [&](unsigned grid, cudaStream_t st) {
+        integrandOpKernel<<<grid, 256, 0, st>>>(op, a, b, out, n);
     });
 }

@@ -453,6 +453,13 @@ int ccoil_eval_log64(const double *x, double *out, long long n, void *stream);
  * op 3 be positive, normal and finite.  Synchronous on `stream`. */
 int ccoil_eval_fp64_op(int op, const double *a, const double *b, double *out, long long n, void *stream);
 
+/* Likewise the roots, reciprocals and quotients of the FP64 integrands.  op 0:
+ * out[i] = sqrt(a[i]); 1: 1 / sqrt(a[i]), the reciprocal of the rounded root (both as the
+ * gradient takes them); 2 and 3: the same as the other integrands take them; 4: a[i] /
+ * sqrt(b[i]) (likewise; b unused and may be NULL for the others); 5: 1 / a[i].  Arguments
+ * of roots and a in op 5 must lie in [1e-36, 1e36], a in op 4 be finite. */
+int ccoil_eval_integrand_op(int op, const double *a, const double *b, double *out, long long n, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -108,3 +108,54 @@ def test_log_ratio64_within_four_ulp(ccoil):
     ref = _extended_ref(np.where(near, np.log1p(np.where(near, (nl - dl) / dl, 0.0)), np.log(q)))
     e = ulp_error(_fp64_op(ccoil, 3, num, den), ref)
     assert e.max() <= 4.0, (e.max(), num[np.argmax(e)], den[np.argmax(e)])
+
+
+def _integrand_op(ccoil, op, a, b=None):
+    import torch
+    ad = torch.from_numpy(a).cuda()
+    bd = torch.from_numpy(b).cuda() if b is not None else None
+    out = torch.empty_like(ad)
+    assert ccoil.lib().ccoil_eval_integrand_op(op, ad.data_ptr(), bd.data_ptr() if bd is not None else None,
+                                               out.data_ptr(), len(a), None) == 0
+    return out.cpu().numpy()
+
+
+def _integrand_args(seed):
+    rng = np.random.default_rng(seed)
+    return np.concatenate([_roots_args(seed), np.exp(rng.uniform(np.log(1e-36), np.log(1e36), 1000000)),
+                           rng.uniform(1e-4, 10.0, 1000000), rng.uniform(1.0, 4.0, 1000000)])
+
+
+@pytest.mark.parametrize("op", [0, 1])
+def test_gradient_roots_equal_ieee(ccoil, op):
+    # root64 and the reciprocal of its root, against the host's IEEE operations: equal
+    x = _integrand_args(53)
+    want = np.sqrt(x) if op == 0 else 1.0 / np.sqrt(x)
+    assert np.array_equal(_integrand_op(ccoil, op, x), want)
+
+
+@pytest.mark.parametrize("op", [2, 3, 4])
+def test_integrand_roots_round_as_ieee_but_for_a_few(ccoil, op):
+    # root64n: a root is within 0.5 ulp + 2^-24 ulp, so 2^-23 of them (0.4 of these 3.3e6)
+    # may round the other way; a reciprocal or quotient follows its root.  Bars: one ulp, and
+    # 10 of them
+    x = _integrand_args(54)
+    n = np.random.default_rng(55).normal(size=len(x))
+    want = np.sqrt(x) if op == 2 else 1.0 / np.sqrt(x) if op == 3 else n / np.sqrt(x)
+    got = _integrand_op(ccoil, op, x) if op < 4 else _integrand_op(ccoil, op, n, x)
+    assert ulp_error(got, want).max() <= 1.0
+    assert np.count_nonzero(got != want) <= 10, np.count_nonzero(got != want)
+
+
+def test_reciprocal_within_one_ulp(ccoil):
+    x = _integrand_args(56)
+    ref = _extended_ref(1 / x.astype(np.longdouble))
+    assert ulp_error(_integrand_op(ccoil, 5, x), ref).max() <= 1.0
+
+
+def test_integrand_op_arguments(ccoil):
+    L = ccoil.lib()
+    assert L.ccoil_eval_integrand_op(6, None, None, None, 0, None) == 1
+    assert L.ccoil_eval_integrand_op(-1, None, None, None, 0, None) == 1
+    assert L.ccoil_eval_integrand_op(0, None, None, None, 4, None) == 1
+    assert L.ccoil_eval_integrand_op(0, None, None, None, 0, None) == 0
