@@ -188,12 +188,15 @@ __device__ __forceinline__ void batchListPoint(const BatchItem &I, const unsigne
 }
 
 // Lists the near-field pairs: a block per item of the lowest field, a thread per point,
-// or, for many segments, a warp (a system of 64 coils at 64 points, the whole call: 247
-// us with threads, 178 with warps).
+// or, for many segments at few points in all (warps), a warp.  The whole call with
+// threads and with warps: one system of 64 coils at 64 points 247 and 178 us, 20 of 32
+// coils at 64 points 244 and 220 us, at 3,000 points 797 and 793 us; 2,048 systems with
+// 24.7 million points 2,276 and 2,284 ms.
 __global__ void __launch_bounds__(128) batchNearListKernel(const unsigned char *__restrict__ blob,
                                                            const SegmentDesc *__restrict__ segs,
                                                            const BatchItem *__restrict__ items, int nitems,
-                                                           int fieldsMask, const double *__restrict__ points,
+                                                           int fieldsMask, bool warps,
+                                                           const double *__restrict__ points,
                                                            NearPair *__restrict__ work,
                                                            unsigned long long workCapacity,
                                                            unsigned long long *__restrict__ workCount)
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(128) batchNearListKernel(const unsigned char *
         const BatchItem I = items[it];
         if (I.field != lowest)
             continue;
-        if (I.seg_end - I.seg_begin >= 16)
+        if (warps && I.seg_end - I.seg_begin >= 16)
             for (int local = threadIdx.x / 32; local < I.point_count; local += 4)
                 batchListPoint<32>(I, blob, segs, fieldsMask, points, local, threadIdx.x % 32, work, workCapacity,
                                    workCount);
@@ -349,7 +352,8 @@ int launchBatchImpl(const BatchLaunch &B, cudaStream_t st)
     if (e == cudaSuccess && B.precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {
         batchNearListKernel<<<(unsigned)std::min(B.nitems, 148 * 64), 128, 0, st>>>(
-            B.d_blob, B.d_segs, items, B.nitems, B.fields_mask, B.d_points, work, B.near.capacity, B.d_work_count);
+            B.d_blob, B.d_segs, items, B.nitems, B.fields_mask, B.points <= (1 << 15), B.d_points, work,
+            B.near.capacity, B.d_work_count);
         batchNearKernel<<<148 * 8, 256, 0, st>>>(B.d_blob, B.d_segs, items, B.nitems, B.d_points, B.d_outA, B.d_outB,
                                                  B.d_outG, work, B.near.contrib, B.near_width, B.near.capacity,
                                                  B.d_work_count);

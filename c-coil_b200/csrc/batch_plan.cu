@@ -150,6 +150,7 @@ BatchLaunch launchOf(ccoil_batch_plan *P, const double *pts, double *a, double *
     B.d_outG = g;
     B.precision = P->precision;
     B.fields_mask = P->fields_mask;
+    B.points = P->points;
     B.grid = P->grid;
     if (P->precision == CCOIL_PRECISION_FP32_COMPENSATED)
     {

@@ -269,6 +269,7 @@ struct BatchLaunch
     double *d_outA, *d_outB, *d_outG;
     int precision;
     int fields_mask;  // bits 1 << CCOIL_FIELD_A, _B, _G
+    long long points;  // of all systems
     int grid;
     void *d_work = nullptr;    // NearPair[near.capacity]
     unsigned long long *d_work_count = nullptr;
