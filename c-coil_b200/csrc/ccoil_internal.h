@@ -191,8 +191,10 @@ struct NearScratch
 // Plans list at most this many: 8 MiB of list, 24 MiB of contributions (72 MiB for the
 // gradient).  The benchmark's groups have 0.07 to 0.4 pairs per point; with more than
 // these a warp per point fills the machine, unless fewer than 9,472 points lie in more
-// than 110 boxes each.  Batch plans a quarter.
-constexpr unsigned long long kNearListPairs = 1ULL << 20, kBatchListPairs = 1ULL << 18;
+// than 110 boxes each.
+constexpr unsigned long long kNearListPairs = 1ULL << 20;
+// batch plans (batch_plan.cu): 2 MiB of list and 6 or 18 of contributions to 8 times that
+constexpr unsigned long long kBatchListMin = 1ULL << 18, kBatchListMax = 1ULL << 21;
 
 // kernels (fields.cu)
 struct FieldLaunch
