@@ -167,7 +167,10 @@ def _evaluate(coil_structs, points, field, precision, lanes=0, stream=None):
 
 
 class FieldPlan:
-    """A prepared coil set (ccoil_field_plan_t): node tables resident in device memory."""
+    """A prepared coil set (ccoil_field_plan_t): node tables resident in device memory.
+
+    FP64 calls on CUDA tensors may overlap on several streams; calls in the FP32 modes, or
+    on host arrays, share buffers of the plan, so the caller keeps them in order."""
 
     def __init__(self, coil_structs, field, precision=PrecisionMode.FP64):
         n = len(coil_structs)

@@ -22,7 +22,8 @@ namespace
 thread_local char t_error[512] = "";
 
 // Grow-only device buffer owned by a plan.  A plan that a user keeps serves any
-// stream, so its buffers are allocated and replaced with the device idle; the plan
+// stream (calls that use its buffers one after the other), so these are allocated
+// and replaced with the device idle; the plan
 // of a one-shot call (scoped) has its buffers in the order of the call's stream.
 struct BufferOwner
 {
@@ -398,9 +399,9 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
         L.d_points = static_cast<const double *>(plan->sortedPoints.ptr);
         L.d_out = static_cast<double *>(plan->sortedOut.ptr);
     }
-    // the pieces' sums: memory of this call alone (a plan may run on several streams
-    // at once), in the order of the stream.  Without it the points are evaluated in
-    // one piece
+    // the pieces' sums: memory of this call alone (FP64 calls of one plan may overlap
+    // on several streams), in the order of the stream.  Without it the points are
+    // evaluated in one piece
     void *partial = nullptr;
     if (pieced)
     {

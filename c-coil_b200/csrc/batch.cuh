@@ -113,9 +113,9 @@ __device__ __forceinline__ void batchItemLanes(const BatchItem &I, const unsigne
 
 // CTAs per SM the register allocation targets, per precision.  FP64: 3
 // (168 registers, no spills; 18.7 ms for B + G over 40 systems of up to 64 coils
-// and 16,384 points, against 20.6 ms at 4 and 23.0 ms at 5).  FP32: 4
-// (128 registers, no spills) measured best for B + G over 2,048 systems on
-// B200: 2.00 s per step against 2.29 s at 5 and 2.54 s at 6
+// and 16,384 points, against 20.6 ms at 4 and 23.0 ms at 5).  FP32: 4 (128
+// registers, no spills): B + G over 2,048 systems 2.28 s per step, 2.39 s at 5 and
+// 2.43 s at 6; 3, at 2.22 s, was found since
 #ifndef CCOIL_BATCH_MIN_BLOCKS
 #define CCOIL_BATCH_MIN_BLOCKS 3
 #endif

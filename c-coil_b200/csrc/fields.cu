@@ -325,7 +325,9 @@ cudaError_t launchField(const FieldLaunch &L, cudaStream_t st)
     // near-field pairs in FP64; the grid loops over the device-side count, so no
     // host synchronisation is needed between the passes
     // few points and many segments: a warp per point (84 segments, 2,797 points: 10 us
-    // against 70)
+    // against 70).  Whole FP32_COMPENSATED B calls at PrecisionFactor 2 with a thread and
+    // with a warp: 16 segments at 100 points 31.6 and 25.7 us, at 16,383 141 and 137 us,
+    // 128 segments at 32,768 points 1,520 and 1,479 us, at 131,072 2,914 and 2,967 us
     // With few pairs the near-field kernel adds up each point's itself, which saves a
     // launch (24 coils, 300 points: 1.6 of 45 us) but costs every warp a fence and an
     // atomic (70 thin coils, 30,000 points, 420,000 pairs: 1,546 against 1,200 us)

@@ -114,12 +114,18 @@ __device__ __forceinline__ Frame toCoilFrame(const SegmentHeader &h, double px, 
 // ---------------------------------------------------------------------------
 // FP64 segment integrals (cylindrical partial sums for one segment)
 //
-// Each node's value is computed with the reference's exact sequence of IEEE
-// double operations (round-to-nearest multiply/add/divide/sqrt, evaluated left
-// to right, no fused multiply-add), because several integrands cancel
-// catastrophically inside a node (e + d for d << 0 in A, G2 - G1 in B, the RZ
-// bracket of G): any other rounding would be amplified far above 1e-12 there.
-// Only the weighting and the accumulation are reassociated.
+// Several integrands cancel catastrophically inside a node (e + d for d << 0 in
+// A, G2 - G1 in B, the RZ bracket of G), and what is in front of such a
+// cancellation would show any other rounding amplified far above 1e-12.  There
+// the reference's order of operations is kept, each rounded by itself:
+// multiplications, additions and subtractions without contraction (mul, add,
+// sub), roots and reciprocals as IEEE operations round, in G always (root64), in
+// A, B and the slow sums but for about one in 10^8 (root64n).  What only scales a
+// node's term need not be: A's logarithm is that of a ratio without its rounded
+// quotient (logRatio64, a few ulp), B's fast quotient is within 0.5 ulp + 2^-26
+// ulp (div64u), G's 1 / M^2 comes from a reciprocal within an ulp (rcp64u),
+// constant factors are taken out of the loops, and the weighting and the
+// accumulation are reassociated and fused.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
@@ -127,9 +133,9 @@ __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, 
 __device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ double sqr(double a) { return __dsqrt_rn(a); }
 
-// The angular loops take roots, reciprocals and quotients from fp64ops.cuh,
-// which equal the IEEE operations bit for bit inside [kLo64, kHi64] at about
-// half their FP64-pipe cost; that pipe bounds every kernel built on these
+// The angular loops take roots, reciprocals and quotients from fp64ops.cuh, at
+// about half the FP64-pipe cost of the compiler's IEEE operations, for arguments
+// in [kLo64, kHi64]; that pipe bounds every kernel built on these
 // integrands.  Whether a thickness node's arguments stay inside is decided
 // once per node from bounds of them (base - k and base + k for base - k c,
 // |c| <= 1: rounding is monotone).  The nodes that do not (a point on a winding

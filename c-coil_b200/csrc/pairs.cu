@@ -14,11 +14,15 @@
 // FP64 (integrands64.cuh), or FP32-compensated (integrands32.cuh) with FP64
 // for secondary nodes in the primary's near-field box.
 //
-// Mapping.  One warp per arrangement (grid-stride); the 32 lanes split the
-// secondary's nodes, each lane evaluates the primary's whole quadrature at its
-// node; the node tables are read from global memory (all lanes read the same
-// primary node: L1 broadcast).  A fixed-order shuffle reduction per primary
-// gives a deterministic result; primaries of a group are summed in order.
+// Mapping.  One warp per work unit (grid-stride): an arrangement, or, of few
+// arrangements, a group of its primaries and a range of its secondary's nodes
+// (PairSplit), which a second kernel adds up.  The 32 lanes split the unit's
+// secondary nodes, each lane, or below a wave of units each 8 neighbouring lanes,
+// evaluating the primary's whole quadrature at its node; FP32_REFINED gives few
+// arrangements a CTA of 4 or 12 warps each instead.  One primary's node tables
+// are staged in shared memory where they fit, others are read from global memory
+// (all lanes read the same primary node: L1 broadcast).  Every sum has a fixed
+// order: results repeat exactly.
 #include "ccoil_internal.h"
 
 #include <cuda_runtime.h>
@@ -1465,7 +1469,7 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
         const PairHeader *ph = reinterpret_cast<const PairHeader *>(blob.data() + off);
         secNodes = std::max(secNodes, ph->s_nl * ph->s_nt * ph->s_na);
     }
-    // work units (the refining kernel needs a primary's whole total in one warp)
+    // work units (the refining kernel needs a primary's whole total in one warp or CTA)
     const long long resident = 148LL * 4 * pairMinBlocks(quantity, fp32, refine);
     PairSplit split;
     int lanes = 1;
@@ -1481,9 +1485,10 @@ int ccoil::pairArrangements(const ccoil_coil_t *primaries, int primary_count, co
     }
     // the refining kernel shares few arrangements among the warps of a CTA: 12 while
     // every arrangement then has a resident CTA, else 4 up to three waves of whole
-    // arrangements (M of 1, 444, 2,000, 8,000 and 32,768 arrangements with one warp
-    // each 0.40, 1.33, 1.73, 2.95 and 9.4 ms, with 4 or 12 0.11, 0.44, 0.93, 2.69 and
-    // 9.9: each warp's last FP64 batch of 32 nodes is partly empty)
+    // arrangements (each warp's last FP64 batch of 32 nodes is partly empty).  Whole
+    // calls with 1, 4 and 12 warps: M of 445 arrangements 1.36, 0.53 and 0.38 ms, 2,000
+    // 1.62, 0.98 and 0.96, 15,984 5.28, 5.22 and 6.04, 20,000 6.35, 6.54 and 7.58; F/T of
+    // 1,000 0.94, 0.46 and 0.40 ms, 2,000 1.14, 0.70 and 0.67, 20,000 4.79, 4.47 and 5.14
     const int team = !refine ? 1 : count <= 148LL * 3 ? 12 : count <= resident * 3 ? 4 : 1;
     const long long perArr = (long long)split.groups * split.parts;
     const size_t atPartial = region(perArr > 1 ? sizeof(double) * (size_t)width * (size_t)(count * perArr) : 0);

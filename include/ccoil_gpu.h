@@ -170,7 +170,12 @@ typedef struct ccoil_field_plan ccoil_field_plan_t;
 
 int ccoil_field_plan_create(const ccoil_coil_t *coils, int coil_count, int field, int precision,
                             ccoil_field_plan_t **plan);
-/* lanes_per_point: 0 = automatic, else 1, 2, 4, 8, 16 or 32 threads share one point. */
+/* lanes_per_point: 0 = automatic, else 1, 2, 4, 8, 16 or 32 threads share one point.
+ * FP64 calls on device memory only read the plan and may overlap on several streams
+ * and host threads.  Calls in the FP32 modes, and calls on host memory, use buffers of
+ * the plan (ordered points, lists, contributions; the device copies of points and
+ * results): the caller orders those of one plan, on one stream or by events, or makes a
+ * plan for each stream. */
 int ccoil_field_plan_execute(ccoil_field_plan_t *plan, const double *points, long long point_count, double *out,
                              int memory, int lanes_per_point, void *stream);
 int ccoil_field_plan_destroy(ccoil_field_plan_t *plan);
