@@ -379,7 +379,7 @@ def bench_batched(a):
                        "points": sum(len(p) for _, p in systems), "coil_points_per_field": coil_points,
                        "precision_factor": a.pf, "l2": "flushed between timed steps (256 MiB write)"},
             "precision_mode": "fp32c", "fp64": res["fp64"], "fp32c": res["fp32c"], "clocks": head["clocks"],
-            "gpu_launches": 2 * a.steps, "host_build_s": build_s}
+            "gpu_launches": 4 * a.steps, "host_build_s": build_s}
     print(json.dumps(line))
 
 
@@ -900,7 +900,8 @@ def ctypes_rates(cc):
 def field_launches(mode, points, segments, field):
     """Kernel launches of one field-plan evaluation (one lane per point): the field kernel and,
     where it is cut into pieces (fewer than 24 waves of 128-point tiles), their sum; in the
-    FP32 modes also the near-field listing and its FP64 pass, and from 16,384 to 2^30 points
+    FP32 modes also the near-field listing, its FP64 pass and, above 2^15 (point, segment)
+    pairs, the sums of each point's pairs, and from 16,384 to 2^30 points
     the point ordering (bounds, Morton keys, the radix sort's 6 kernels, gather) and the
     scatter of the results; FP32_REFINED per chunk of points (contributions of at most
     4 GiB, at most 2^28 listed pairs) also the selection (count, scan, select) and FP64 pair
@@ -914,12 +915,17 @@ def field_launches(mode, points, segments, field):
     if mode == 0:
         return 1 + sums(points)
     ordering = 10 if (1 << 14) <= points <= (1 << 30) else 0
+
+    def near(n):
+        return 3 if n * segments > 1 << 15 else 2
+
     if mode == 1:
-        return 3 + sums(points) + ordering
+        return 1 + near(points) + sums(points) + ordering
     width = 9 if field == 3 else 3
     per_chunk = min((1 << 32) // (segments * width * 8), (1 << 28) // segments)
     chunks = -(-points // max(1, per_chunk))
-    return ordering + (7 + sums(-(-points // chunks))) * chunks
+    per_chunk = -(-points // chunks)
+    return ordering + (5 + near(per_chunk) + sums(per_chunk)) * chunks
 
 
 def read_profile(field, mode):

@@ -562,7 +562,7 @@ __device__ __forceinline__ void integrateSegmentRefine(const unsigned char *seg,
 // count (this pass for A of 15 coils at 389 points, 1,500 pairs: 263 us with one
 // thread per pair, 59 us with 32).
 // CTAs per SM of the FP64 pair pass: several nodes in flight per thread without
-// spills (vector potential 120 registers, field 112, gradient 142) measured 1 %
+// spills (vector potential and field 120 registers, gradient 152) measured 1 %
 // faster for the whole call than the most CTAs that fit without (6, 5 and 4)
 constexpr int refineMinBlocks(int field) { return field == CCOIL_FIELD_G ? 3 : 4; }
 template <int FIELD, int LANES>

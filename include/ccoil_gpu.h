@@ -412,7 +412,9 @@ int ccoil_inject_allocation_failures(int count);
  *
  * Its scratch (node tables, segment list, near-field work list) is one fixed
  * 3 MiB array in device memory, held by every GPU that loads the library until
- * the process exits.  Limits: at most 1 MiB of node tables (about 400 coils at
+ * the process exits.  The list has room for 53,248 (point, segment) pairs, for
+ * the gradient 21,299; with more, the points are searched for them again.
+ * Limits: at most 1 MiB of node tables (about 400 coils at
  * PrecisionFactor 5), 8192 segments and 2^31-1 points; larger requests return
  * CCOIL_ERR_INVALID_ARGUMENT with a message.  A call on a stream that is being
  * captured returns CCOIL_ERR_NOT_SUPPORTED: every call stages the node tables
