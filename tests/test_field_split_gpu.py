@@ -250,3 +250,28 @@ def test_batch_overflow_with_segments_shared_in_a_warp(ccoil):
             want = ccoil.FieldPlan([c.struct() for c in coils], field, ccoil.PrecisionMode.FP32_COMPENSATED)(pts)
             assert rel_err(got[f].cpu().numpy(), want).max() < TOL, (f, n)
         batch.close()
+
+
+@pytest.mark.parametrize("mode", ["FP32_COMPENSATED", "FP32_REFINED"])
+@pytest.mark.parametrize("field", [0, 1, 3])
+@pytest.mark.parametrize("points", [37, 3001])
+def test_captured_fp32_call_repeats(ccoil, mode, field, points):
+    # the near-field list's counter is cleared by a kernel or a memset of the call: each
+    # replay starts from an empty list.  The pieces that an eager call is cut into add in
+    # another order (bar of test_pieces_match_captured_call; FP32_REFINED may pick another
+    # pair at its threshold, as in test_pair_split_gpu.py: 1e-7)
+    import torch
+    plan = ccoil.FieldPlan([c.struct() for c in stack(ccoil, 40)], field, ccoil.PrecisionMode[mode])
+    x = torch.from_numpy(on_the_winding(points, 0.02)).cuda()
+    eager = plan(x).cpu().numpy()
+    out = torch.empty((points, plan.width), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        plan(x, out=out)
+    for _ in range(3):
+        out.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        assert rel_err(out.cpu().numpy(), eager).max() < (TOL if mode == "FP32_COMPENSATED" else 1e-7)
+    plan.close()
