@@ -343,13 +343,21 @@ int runFields(ccoil_field_plan *plan, const double *dPoints, long long point_cou
     if (plan->precision == CCOIL_PRECISION_FP32_COMPENSATED || plan->precision == CCOIL_PRECISION_FP32_REFINED)
     {
         // near-field work list: room for every (point, segment) pair up to
-        // kNearListPairs (with more near-field pairs the near-field pass finds them
+        // kNearListPairs, for few points kNearListPairsFewPoints (with more near-field pairs the near-field pass finds them
         // itself; FP32_REFINED's selection: every pair of a chunk, up to
         // kRefineListPairs), and after it what else the near-field pass needs
         const unsigned long long want = std::max(1ULL, (unsigned long long)chunk * (unsigned long long)L.nseg);
-        const unsigned long long cap = std::min(want, refined ? kRefineListPairs : kNearListPairs);
-        const unsigned long long near = std::min(want, kNearListPairs);
-        int rc0 = plan->work.reserve(cap * kNearPairBytes + NearScratch::bytes(near, width), plan->owner);
+        unsigned long long near =
+            std::min(want, chunk <= kNearFewPoints ? kNearListPairsFewPoints : kNearListPairs);
+        auto bytes = [&] {
+            return (refined ? std::min(want, kRefineListPairs) : near) * kNearPairBytes + NearScratch::bytes(near, width);
+        };
+        // a captured call allocates nothing: it takes the buffer of an earlier call of at
+        // least as many points, which may have had the short list
+        if (capture != cudaStreamCaptureStatusNone && bytes() > plan->work.bytes)
+            near = std::min(want, kNearListPairs);
+        const unsigned long long cap = refined ? std::min(want, kRefineListPairs) : near;
+        int rc0 = plan->work.reserve(bytes(), plan->owner);
         if (rc0 == CCOIL_OK)
             rc0 = plan->workCount.reserve(sizeof(unsigned long long), plan->owner);
         if (rc0 != CCOIL_OK)

@@ -265,7 +265,10 @@ int ccoil_batch_plan_create(const ccoil_coil_t *coils, const int *system_coil_of
         for (int f = CCOIL_FIELD_A; f <= CCOIL_FIELD_G; ++f)
             fields += (fields_mask >> f) & 1;
         all *= (unsigned long long)fields;
-        P->nearPairs = std::max(1ULL, std::min(all, std::clamp(all / 64, kBatchListMin, kBatchListMax)));
+        // (few points: as in the field plans)
+        P->nearPairs = std::max(1ULL, std::min(all, npts * fields <= kNearFewPoints
+                                                        ? kNearListPairsFewPoints
+                                                        : std::clamp(all / 64, kBatchListMin, kBatchListMax)));
         rc = P->work.reserve(kNearPairBytes * P->nearPairs +
                              NearScratch::bytes(P->nearPairs, fields_mask & (1 << CCOIL_FIELD_G) ? 9 : 3));
         if (rc == CCOIL_OK)

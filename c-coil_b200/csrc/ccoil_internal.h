@@ -190,9 +190,11 @@ struct NearScratch
 };
 // Plans list at most this many: 8 MiB of list, 24 MiB of contributions (72 MiB for the
 // gradient).  The benchmark's groups have 0.07 to 0.4 pairs per point; with more than
-// these a warp per point fills the machine, unless fewer than 9,472 points lie in more
-// than 110 boxes each.
-constexpr unsigned long long kNearListPairs = 1ULL << 20;
+// these a warp per point fills the machine.  Up to 9,472 points, the warps that run at
+// once, it would not: there the list is up to 4 times as long.  B of 320 coils in one
+// place at 4,000 points, 1.28 million pairs: 10.6 ms with the short list, 8.9 with the long.
+constexpr unsigned long long kNearListPairs = 1ULL << 20, kNearListPairsFewPoints = 1ULL << 22;
+constexpr long long kNearFewPoints = 148 * 64;
 // batch plans (batch_plan.cu): 2 MiB of list and 6 or 18 of contributions to 8 times that
 constexpr unsigned long long kBatchListMin = 1ULL << 18, kBatchListMax = 1ULL << 21;
 

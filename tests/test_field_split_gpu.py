@@ -236,12 +236,13 @@ def test_pairs_of_one_point_run_side_by_side(ccoil):
 
 
 def test_batch_overflow_with_segments_shared_in_a_warp(ccoil):
-    # 33 coils in one place: listed a warp per point; 4,100 points give 270,600 pairs over
-    # two fields, more than the list's 2^18, and 3,900 points 257,400, fewer.  Every pair is
-    # FP64, so the plan's sums, in the same order
+    # 33 coils in one place: listed a warp per point.  3,900 and 4,100 points give 257,400
+    # and 270,600 pairs over two fields, all listed; 4,800 points, above the bound for few
+    # points, 316,800, more than the list's 2^18.  Every pair is FP64, so the plan's sums,
+    # in the same order
     coils = [ccoil.Coil(0.1, 0.02, 0.05, 10 + i, 1.0 + i) for i in range(33)]
     g = np.random.default_rng(9)
-    for n in (3900, 4100):
+    for n in (3900, 4100, 4800):
         r, phi = g.uniform(0.095, 0.125, n), g.uniform(0.0, 2.0 * np.pi, n)
         pts = np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, n)], axis=1)
         batch = ccoil.BatchPlan([(coils, pts)], fields=("A", "B"), precision=ccoil.PrecisionMode.FP32_COMPENSATED)
@@ -274,4 +275,28 @@ def test_captured_fp32_call_repeats(ccoil, mode, field, points):
         g.replay()
         torch.cuda.synchronize()
         assert rel_err(out.cpu().numpy(), eager).max() < (TOL if mode == "FP32_COMPENSATED" else 1e-7)
+    plan.close()
+
+
+def test_few_points_captured_after_many(ccoil):
+    # 130 coils in one place: 9,000 points may list 1.17 million pairs, 12,000 points 2^20;
+    # a call of 12,000 points has reserved enough for a captured one of 9,000.  Every pair is
+    # FP64 and added in the same order, listed or not
+    import torch
+    coils = [ccoil.Coil(0.1, 0.0, 0.05, 10 + i, 1.0 + i) for i in range(130)]
+    g = np.random.default_rng(10)
+    r, phi = g.uniform(0.095, 0.105, 12000), g.uniform(0.0, 2.0 * np.pi, 12000)
+    x = torch.from_numpy(np.stack([r * np.cos(phi), r * np.sin(phi), g.uniform(-0.03, 0.03, 12000)], axis=1)).cuda()
+    plan = ccoil.FieldPlan([c.struct() for c in coils], 1, ccoil.PrecisionMode.FP32_COMPENSATED)
+    whole = plan(x)
+    out = torch.empty((9000, 3), dtype=torch.float64, device="cuda")
+    y = x[:9000].contiguous()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan(y, out=out)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, whole[:9000])
+    assert torch.equal(plan(y), out)
     plan.close()
